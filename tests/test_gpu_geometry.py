@@ -68,3 +68,32 @@ def test_winding_invariance_on_gpu():
     a = voxelize(mesh, None, (64, 64, 64), False)
     b = voxelize(meshes.Mesh(rev, mesh.triangle_count), None, (64, 64, 64), False)
     assert a.solid_cells == 64 and np.array_equal(a.geometry, b.geometry)
+
+
+# triangle counts around the warp's 32 (few triangles: their pixels split over many
+# warps), boxes of many pixels and of none, a grid that is odd in every direction
+@pytest.mark.parametrize("floor", [False, True])
+@pytest.mark.parametrize("name,make", [
+    ("12 large", lambda: box([3.2, 4.7, 2.9], [30.1, 25.3, 19.8])),
+    ("20", lambda: meshes.icosphere((15.3, 14.1, 11.2), 8.7, 0)),
+    ("32", lambda: meshes.icosphere((15.3, 14.1, 11.2), 8.7, 0, 4)),
+    ("35", lambda: meshes.icosphere((15.3, 14.1, 11.2), 8.7, 0, 5)),
+    ("1280", lambda: meshes.icosphere((15.3, 14.1, 11.2), 8.7, 3)),
+    ("outside", lambda: box([-9.5, -3.5, 30.2], [60.5, 2.5, 44.1])),
+])
+def test_voxelizer_triangle_groups(name, make, floor):
+    g, r = _both(make(), None, (37, 29, 23), floor)
+    assert np.array_equal(g.geometry, r.geometry)
+    assert np.array_equal(g.boundary_cells, r.boundary_cells)
+    assert (g.solid_cells, g.frontal_cells, g.watertight) == (r.solid_cells, r.frontal_cells, r.watertight)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("at", [0, 8, -1])
+def test_voxelizer_rejects_non_finite_body(value, at):
+    from pocketwind_gb300._lib import RangeError
+    from pocketwind_gb300.geometry import voxelize
+    bad = meshes.icosphere((16, 16, 16), 8, 1).positions.copy()
+    bad[at] = value
+    with pytest.raises(RangeError):
+        voxelize(bad, None, (32, 32, 32), False)
