@@ -120,11 +120,13 @@ __global__ void __launch_bounds__(kScanThreads) scan_sums(const uint32_t *in, ui
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// One block: the exclusive scan of the block sums in place; the total to *total_a and *total_b.
+// One block an array of block sums (array b at sums + b * blocks): its exclusive scan in
+// place; its total to total_a[b] and total_b[b].
 __global__ void __launch_bounds__(kScanThreads) scan_offsets(uint32_t *sums, uint32_t blocks, uint32_t *total_a,
                                                             uint32_t *total_b) {
   __shared__ uint32_t warps[33];
   uint32_t carry = 0;
+  sums += (size_t)blockIdx.x * blocks;
   for (uint32_t base = 0; base < blocks; base += kScanThreads) {
     const uint32_t i = base + threadIdx.x;
     const uint32_t v = i < blocks ? sums[i] : 0u;
@@ -135,8 +137,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_offsets(uint32_t *sums, uin
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    *total_a = carry;
-    if (total_b) *total_b = carry;
+    total_a[blockIdx.x] = carry;
+    if (total_b) total_b[blockIdx.x] = carry;
   }
 }
 
@@ -336,85 +338,134 @@ __global__ void __launch_bounds__(128) column_kernel(Proj P, const uint32_t *off
   }
 }
 
-__global__ void classify_kernel(const uint8_t *votes, uint32_t *flags, size_t cells, uint32_t type) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < cells && votes[i] >= 2 && flags[i] == pw::FLUID) flags[i] = type;
+// Every cell's kind from the meshes' votes (two of the three projections; body
+// before supports), then the boundary planes (voxelize.ts:123-135: the floor
+// plane, the top plane over a floor, the x faces), and countCells
+// (voxelize.ts:137-154): solid cells, and the (y, z) rows that hold one.
+// body or sup is null without such a mesh.
+__global__ void kinds_kernel(const uint8_t *body, const uint8_t *sup, uint32_t *flags, uint32_t nx, uint32_t ny,
+                             uint32_t nz, int floor_on, uint32_t *solid, uint8_t *body_rows, uint8_t *wall_rows) {
+  const size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool in = at < (size_t)nx * ny * nz;
+  const uint32_t i = (uint32_t)at, row = i / nx, x = i - row * nx, z = row / ny;
+  uint32_t t = pw::FLUID;
+  if (in) {
+    if (body && body[at] >= 2) t = pw::SOLID;
+    else if (sup && sup[at] >= 2) t = pw::SUPPORT;
+    if (floor_on && z == 0) t = pw::FLOOR;
+    else if (floor_on && z == nz - 1) t = pw::EQ;
+    else if (x == 0 || x == nx - 1) t = pw::EQ;
+    flags[at] = t;
+    if (t == pw::SOLID) body_rows[row] = 1;
+    if (t == pw::SOLID || t == pw::SUPPORT) wall_rows[row] = 1;
+  }
+  const uint32_t n = __popc(__ballot_sync(0xffffffffu, in && t == pw::SOLID));
+  if (n && (threadIdx.x & 31u) == 0u) atomicAdd(solid, n);
 }
 
-// voxelize.ts:123-135 (x faces, then the floor plane and the top plane)
-__global__ void boundary_kernel(uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, int floor_on) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t cells = (size_t)nx * ny * nz;
-  if (i >= cells) return;
-  uint32_t x = (uint32_t)(i % nx);
-  uint32_t z = (uint32_t)(i / ((size_t)nx * ny));
-  if (floor_on && z == 0) flags[i] = pw::FLOOR;
-  else if (floor_on && z == nz - 1) flags[i] = pw::EQ;
-  else if (x == 0 || x == nx - 1) flags[i] = pw::EQ;
-}
-
-// countCells, voxelize.ts:137-154
-__global__ void count_kernel(const uint32_t *flags, size_t cells, uint32_t nx, uint32_t *solid,
-                             uint8_t *body_proj, uint8_t *wall_proj) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cells) return;
-  uint32_t t = flags[i] & 7u;
-  if (t == pw::SOLID) { atomicAdd(solid, 1u); body_proj[i / nx] = 1; }
-  if (t == pw::SOLID || t == pw::SUPPORT) wall_proj[i / nx] = 1;
-}
-
-__global__ void sum_u8_kernel(const uint8_t *v, size_t n, uint32_t *out) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t x = i < n ? v[i] : 0u;
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-  if ((threadIdx.x & 31) == 0 && x) atomicAdd(out, x);
+// The rows marked in each of the two row arrays (one after the other) into out[0] and out[1].
+__global__ void sum_rows_kernel(const uint8_t *v, size_t rows, uint32_t *out) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int a = 0; a < 2; a++) {
+    const uint32_t n = __popc(__ballot_sync(0xffffffffu, i < rows && v[(size_t)a * rows + i] != 0));
+    if (n && (threadIdx.x & 31u) == 0u) atomicAdd(out + a, n);
+  }
 }
 
 // markWalls, wall-links.ts:34-51, gathered per fluid cell: bit (3+i) when the
 // pull source x - c_i (x bounded, y periodic, z bounded with a floor) is a wall.
 // Only fluid words change and their type bits stay, so concurrent readers of a
-// neighbour's type see the same kind before and after its write.
-__global__ void wall_mask_kernel(uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, int floor_on,
-                                 uint32_t *link_count, uint32_t *is_boundary) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t cells = (size_t)nx * ny * nz;
-  if (i >= cells) return;
-  uint32_t f = flags[i];
-  uint32_t mask = 0, body = 0;
-  if ((f & 7u) == pw::FLUID) {
-    long x = (long)(i % nx), y = (long)((i / nx) % ny), z = (long)(i / ((size_t)nx * ny));
+// neighbour's type see the same kind before and after its write.  Fluid cells
+// next to the body also get kBodyBit, until pack_links_kernel takes it out.
+// Each block sums the links and the body's neighbours of its 1,024 cells, all
+// that the packing pass needs of the cells before its own: with 32-bit cell
+// arithmetic and no per-cell counts this pass, the packing pass and their scan
+// take the place of six passes (134 us for the masks alone, with 64-bit
+// remainders, and 103 us for the counts' scans, the q offsets, the fractions
+// and the boundary list, at 256x128x128).
+constexpr uint32_t kBodyBit = 1u << 31;
+constexpr uint32_t kLinkBits = 0x3ffff0u;
+constexpr int kMaskThreads = 256, kMaskCells = 4 * kMaskThreads;
+
+__global__ void __launch_bounds__(kMaskThreads) wall_mask_kernel(uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz,
+                                                                int floor_on, uint32_t *sums, uint32_t blocks) {
+  __shared__ uint32_t total[2];
+  if (threadIdx.x < 2) total[threadIdx.x] = 0u;
+  __syncthreads();
+  const size_t cells = (size_t)nx * ny * nz, base = (size_t)blockIdx.x * kMaskCells + threadIdx.x;
+  const uint32_t plane = nx * ny;
+  uint32_t links = 0, next = 0;
+  for (int k = 0; k < 4; k++) {
+    const size_t at = base + (size_t)k * kMaskThreads;
+    if (at >= cells) break;
+    const uint32_t i = (uint32_t)at, f = flags[at];
+    if ((f & 7u) != pw::FLUID) continue;
+    const uint32_t row = i / nx, x = i - row * nx, z = row / ny, y = row - z * ny;
+    // offsets to the source of each axis' step (mod 2^32, as the cell index)
+    const uint32_t ym = y == 0 ? plane - nx : 0u - nx, yp = y + 1 == ny ? nx - plane : nx;
+    const uint32_t span = plane * nz;
+    const uint32_t zm = z == 0 ? span - plane : 0u - plane, zp = z + 1 == nz ? plane - span : plane;
+    const bool has_xm = x > 0, has_xp = x + 1 < nx, has_zm = !(floor_on && z == 0), has_zp = !(floor_on && z + 1 == nz);
+    uint32_t mask = 0;
+    bool body = false;
 #pragma unroll
     for (int d = 1; d < 19; d++) {
-      long sx = x - pw::cx_of(d), sy = y - pw::cy_of(d), sz = z - pw::cz_of(d);
-      if (sx < 0 || sx >= (long)nx) continue;
-      if (floor_on && (sz < 0 || sz >= (long)nz)) continue;
-      sy = (sy + ny) % ny;
-      sz = (sz + nz) % nz;
-      uint32_t t = flags[(size_t)sx + (size_t)nx * ((size_t)sy + (size_t)ny * (size_t)sz)] & 7u;
-      if (t >= pw::SOLID && t <= pw::FLOOR) {
-        mask |= 1u << (3 + d);
-        if (t == pw::SOLID) body = 1;
-      }
+      const int cx = pw::cx_of(d), cy = pw::cy_of(d), cz = pw::cz_of(d);
+      if ((cx > 0 && !has_xm) || (cx < 0 && !has_xp) || (cz > 0 && !has_zm) || (cz < 0 && !has_zp)) continue;
+      const uint32_t src = i + (cx > 0 ? ~0u : (cx < 0 ? 1u : 0u)) + (cy > 0 ? ym : (cy < 0 ? yp : 0u)) +
+                           (cz > 0 ? zm : (cz < 0 ? zp : 0u));
+      const uint32_t t = flags[src] & 7u;
+      if (t >= pw::SOLID && t <= pw::FLOOR) mask |= 1u << (3 + d);
+      body = body || t == pw::SOLID;
     }
-    if (mask) flags[i] = f | mask;
+    if (mask) flags[at] = f | mask | (body ? kBodyBit : 0u);
+    links += __popc(mask);
+    next += body ? 1u : 0u;
   }
-  link_count[i] = __popc(mask);
-  is_boundary[i] = body;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    links += __shfl_down_sync(0xffffffffu, links, o);
+    next += __shfl_down_sync(0xffffffffu, next, o);
+  }
+  if ((threadIdx.x & 31u) == 0u && links) {
+    atomicAdd(&total[0], links);
+    atomicAdd(&total[1], next);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) sums[(size_t)threadIdx.x * blocks + blockIdx.x] = total[threadIdx.x];
 }
 
-__global__ void qoff_kernel(const uint32_t *link_count, const uint32_t *scan, uint32_t *qoff, size_t cells) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < cells) qoff[i] = link_count[i] ? scan[i] : PW_NO_Q;
-}
-
-__global__ void compact_kernel(const uint32_t *is_boundary, const uint32_t *scan, uint32_t *out, size_t cells) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < cells && is_boundary[i]) out[scan[i]] = (uint32_t)i;
-}
-
-__global__ void fill_float_kernel(float *p, size_t n, float v) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
+// The packed geometry of a block's 1,024 cells: q offsets, halfway fractions and
+// the ascending list of the body's neighbours, from the block's offsets.
+__global__ void __launch_bounds__(kMaskThreads) pack_links_kernel(uint32_t *flags, size_t cells, const uint32_t *offsets,
+                                                                 uint32_t blocks, uint32_t *qoff, float *fractions,
+                                                                 uint32_t *boundary) {
+  __shared__ uint32_t warps[33];
+  uint32_t at_link = offsets[blockIdx.x], at_body = offsets[(size_t)blocks + blockIdx.x];
+  for (int k = 0; k < 4; k++) {
+    const size_t i = (size_t)blockIdx.x * kMaskCells + (size_t)k * kMaskThreads + threadIdx.x;
+    const uint32_t f = i < cells ? flags[i] : 0u;
+    const uint32_t n = __popc(f & kLinkBits), b = f >> 31;
+    uint32_t off = PW_NO_Q;
+    if (__syncthreads_or(n)) {
+      uint32_t sum_n, sum_b;
+      const uint32_t first = at_link + block_scan(n, warps, &sum_n);
+      __syncthreads();
+      const uint32_t rank = at_body + block_scan(b, warps, &sum_b);
+      if (n) {
+        off = first;
+        for (uint32_t r = 0; r < n; r++) fractions[first + r] = 0.5f;
+        if (b) {
+          boundary[rank] = (uint32_t)i;
+          flags[i] = f & ~kBodyBit;
+        }
+      }
+      at_link += sum_n;
+      at_body += sum_b;
+    }
+    if (i < cells) qoff[i] = off;
+  }
 }
 
 static inline unsigned nblk(size_t n, unsigned b = 256) { return (unsigned)((n + b - 1) / b); }
@@ -422,9 +473,10 @@ static inline unsigned nblk(size_t n, unsigned b = 256) { return (unsigned)((n +
 // What the voxelization's kernels report, one copy to the host.
 struct GridInfo {
   uint32_t solid, frontal, blocked;  // countCells
-  uint32_t odd;                      // a column with an odd number of hits: the mesh is open
+  uint32_t odd[2];                   // body, supports: a column with an odd number of hits (an open mesh)
   uint32_t nonfinite;                // a coordinate that is not finite
   uint32_t hits;
+  uint32_t links, boundary;          // wall links; fluid cells next to the body
 };
 
 static int read_info(const GridInfo *info, GridInfo *out, cudaStream_t s) {
@@ -433,8 +485,11 @@ static int read_info(const GridInfo *info, GridInfo *out, cudaStream_t s) {
   return PW_OK;
 }
 
-static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t ny, uint32_t nz,
-                     uint32_t *flags, uint32_t type, bool *watertight, cudaStream_t s) {
+// The votes of one mesh, one byte a cell (null without triangles; the caller's to
+// free).  which: 0 the body, 1 the supports.
+static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t ny, uint32_t nz, int which,
+                     GridInfo *info, uint8_t **votes_out, cudaStream_t s) {
+  if (ntri == 0) return PW_OK;
   const size_t cells = (size_t)nx * ny * nz;
   const uint32_t sizes[3] = {nx, ny, nz};
   const size_t strides[3] = {1, nx, (size_t)nx * ny};
@@ -446,23 +501,19 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
     P.p[p] = Proj{u, v, a, sizes[u], sizes[v], sizes[a], strides[u], strides[v], strides[a], ncol};
     ncol += (size_t)sizes[u] * sizes[v];
   }
-  *watertight = true;
-  if (ntri == 0) return PW_OK;
-  uint8_t *votes = nullptr;
   uint32_t *count = nullptr, *offset = nullptr;
-  GridInfo *info = nullptr, got{};
+  GridInfo got{};
   double *hits = nullptr;
-  cudaError_t e = tmp_alloc(&votes, cells, s);
+  cudaError_t e = tmp_alloc(votes_out, cells, s);
+  uint8_t *votes = *votes_out;
   if (e == cudaSuccess) e = tmp_alloc(&count, ncol * 4, s);
   if (e == cudaSuccess) e = tmp_alloc(&offset, (ncol + 1) * 4, s);
-  if (e == cudaSuccess) e = tmp_alloc(&info, sizeof(GridInfo), s);
   int rc = e == cudaSuccess ? PW_OK : cuda_status(e, "voxelize columns");
   // one warp a group of 32 triangles, or as many as fill the GPU's 152 SMs with 16
   const uint32_t groups = (ntri + 31u) / 32u;
   const uint32_t slices = std::max(1u, std::min(1024u, 152u * 16u / groups));
   const unsigned rblocks = (unsigned)(((uint64_t)groups * slices + kRasterThreads / 32 - 1) / (kRasterThreads / 32));
   if (rc == PW_OK) {
-    cudaMemsetAsync(info, 0, sizeof(GridInfo), s);
     cudaMemsetAsync(votes, 0, cells, s);
     cudaMemsetAsync(count, 0, ncol * 4, s);
     raster_kernel<false><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, nullptr, nullptr,
@@ -480,13 +531,11 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
     if (rc == PW_OK) {
       raster_kernel<true><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, offset, hits, nullptr);
       for (int p = 0; p < 3; p++)
-        column_kernel<<<nblk((size_t)P.p[p].su * P.p[p].sv, 128), 128, 0, s>>>(P.p[p], offset, hits, votes, &info->odd);
-      classify_kernel<<<nblk(cells), 256, 0, s>>>(votes, flags, cells, type);
-      rc = read_info(info, &got, s);
+        column_kernel<<<nblk((size_t)P.p[p].su * P.p[p].sv, 128), 128, 0, s>>>(P.p[p], offset, hits, votes,
+                                                                               &info->odd[which]);
     }
   }
-  *watertight = got.odd == 0;
-  tmp_free(votes, s); tmp_free(count, s); tmp_free(offset, s); tmp_free(info, s); tmp_free(hits, s);
+  tmp_free(count, s); tmp_free(offset, s); tmp_free(hits, s);
   return rc;
 }
 
@@ -705,67 +754,49 @@ static bool finite_mesh(const float *m, uint32_t ntri) {
   return true;
 }
 
-static int read_total(const uint32_t *total, uint32_t *out, cudaStream_t s) {
-  PW_TRY(cudaMemcpyAsync(out, total, 4, cudaMemcpyDeviceToHost, s));
-  PW_TRY(cudaStreamSynchronize(s));
-  return PW_OK;
-}
-
-// Shared tail: wall masks, q offsets, halfway fractions, boundary list, counts.
-static int finish_grid(pw_grid *g, int floor_on, bool body_closed, bool supports_closed, cudaStream_t s) {
-  size_t cells = g->cells;
-  uint32_t *link_count = nullptr, *is_boundary = nullptr, *scan = nullptr, *solid = nullptr;
-  uint8_t *proj = nullptr;
-  size_t plane = (size_t)g->ny * g->nz;
-  cudaError_t e = tmp_alloc(&link_count, cells * 4, s);
-  if (e == cudaSuccess) e = tmp_alloc(&is_boundary, cells * 4, s);
-  if (e == cudaSuccess) e = tmp_alloc(&scan, (cells + 1) * 4, s);
-  if (e == cudaSuccess) e = tmp_alloc(&solid, 16, s);
-  if (e == cudaSuccess) e = tmp_alloc(&proj, 2 * plane, s);
+// From the meshes' votes to the finished grid: kinds, wall masks, q offsets,
+// halfway fractions, boundary list, counts.
+static int finish_grid(pw_grid *g, const uint8_t *body, const uint8_t *sup, int floor_on, GridInfo *info,
+                       cudaStream_t s) {
+  const size_t cells = g->cells, rows = (size_t)g->ny * g->nz;
+  const uint32_t blocks = nblk(cells, kMaskCells);
+  uint32_t *sums = nullptr;
+  uint8_t *marked = nullptr;
+  GridInfo got{};
+  cudaError_t e = tmp_alloc(&sums, 2 * (size_t)blocks * 4, s);
+  if (e == cudaSuccess) e = tmp_alloc(&marked, 2 * rows, s);
+  if (e == cudaSuccess) e = cudaMalloc(&g->qoff, cells * 4);
   int rc = e == cudaSuccess ? PW_OK : cuda_status(e, "voxelize counts");
-  uint32_t counts[4] = {0, 0, 0, 0};
   if (rc == PW_OK) {
-    cudaMemsetAsync(solid, 0, 16, s);
-    cudaMemsetAsync(proj, 0, 2 * plane, s);
-    count_kernel<<<nblk(cells), 256, 0, s>>>(g->flags, cells, g->nx, solid, proj, proj + plane);
-    sum_u8_kernel<<<nblk(plane), 256, 0, s>>>(proj, plane, solid + 1);
-    sum_u8_kernel<<<nblk(plane), 256, 0, s>>>(proj + plane, plane, solid + 2);
-    wall_mask_kernel<<<nblk(cells), 256, 0, s>>>(g->flags, g->nx, g->ny, g->nz, floor_on, link_count, is_boundary);
-    uint32_t nfrac = 0, nb = 0;
-    rc = exclusive_scan(link_count, scan, cells, nullptr, s);
-    if (rc == PW_OK) rc = read_total(scan + cells, &nfrac, s);
-    if (rc == PW_OK) {
-      e = cudaMalloc(&g->qoff, cells * 4);
-      if (e == cudaSuccess) e = cudaMalloc(&g->fractions, ((size_t)nfrac ? nfrac : 1) * 4);
-      if (e != cudaSuccess) rc = cuda_status(e, "voxelize q");
-    }
-    if (rc == PW_OK) {
-      qoff_kernel<<<nblk(cells), 256, 0, s>>>(link_count, scan, g->qoff, cells);
-      if (nfrac) fill_float_kernel<<<nblk(nfrac), 256, 0, s>>>(g->fractions, nfrac, 0.5f);
-      g->nfrac = nfrac;
-      rc = exclusive_scan(is_boundary, scan, cells, nullptr, s);
-    }
-    if (rc == PW_OK) rc = read_total(scan + cells, &nb, s);
-    if (rc == PW_OK) {
-      e = cudaMalloc(&g->boundary, ((size_t)nb ? nb : 1) * 4);
-      if (e != cudaSuccess) rc = cuda_status(e, "voxelize boundary");
-    }
-    if (rc == PW_OK) {
-      compact_kernel<<<nblk(cells), 256, 0, s>>>(is_boundary, scan, g->boundary, cells);
-      g->nboundary = nb;
-      e = cudaMemcpyAsync(counts, solid, 12, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) rc = cuda_status(e, "voxelize finish");
-    }
+    cudaMemsetAsync(marked, 0, 2 * rows, s);
+    kinds_kernel<<<nblk(cells), 256, 0, s>>>(body, sup, g->flags, g->nx, g->ny, g->nz, floor_on, &info->solid, marked,
+                                             marked + rows);
+    sum_rows_kernel<<<nblk(rows), 256, 0, s>>>(marked, rows, &info->frontal);
+    wall_mask_kernel<<<blocks, kMaskThreads, 0, s>>>(g->flags, g->nx, g->ny, g->nz, floor_on, sums, blocks);
+    scan_offsets<<<2, kScanThreads, 0, s>>>(sums, blocks, &info->links, nullptr);
+    rc = read_info(info, &got, s);
   }
-  tmp_free(link_count, s); tmp_free(is_boundary, s); tmp_free(scan, s); tmp_free(solid, s); tmp_free(proj, s);
+  if (rc == PW_OK) {
+    e = cudaMalloc(&g->fractions, ((size_t)got.links ? got.links : 1) * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&g->boundary, ((size_t)got.boundary ? got.boundary : 1) * 4);
+    if (e != cudaSuccess) rc = cuda_status(e, "voxelize links");
+  }
+  if (rc == PW_OK) {
+    pack_links_kernel<<<blocks, kMaskThreads, 0, s>>>(g->flags, cells, sums, blocks, g->qoff, g->fractions,
+                                                      g->boundary);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) rc = cuda_status(e, "voxelize finish");
+  }
+  tmp_free(sums, s); tmp_free(marked, s);
   if (rc != PW_OK) return rc;
+  g->nfrac = got.links;
+  g->nboundary = got.boundary;
   pw_grid_stats &st = g->stats;
   st.nx = g->nx; st.ny = g->ny; st.nz = g->nz;
-  st.solid_cells = counts[0];
-  st.frontal_cells = counts[1];
-  st.blockage = (double)counts[2] / ((double)g->ny * g->nz);
-  st.watertight = body_closed && supports_closed;
+  st.solid_cells = got.solid;
+  st.frontal_cells = got.frontal;
+  st.blockage = (double)got.blocked / ((double)g->ny * g->nz);
+  st.watertight = !got.odd[0] && !got.odd[1];
   st.missed_links = 0;
   st.geometry_len = 2 * (uint64_t)cells + g->nfrac;
   st.boundary_cells = g->nboundary;
@@ -849,30 +880,33 @@ int pw_voxelize_opts(const float *body, uint32_t body_triangles, const float *su
   g->nx = nx; g->ny = ny; g->nz = nz; g->cells = cells;
   float *d_mesh = nullptr;
   int rc = PW_OK;
-  bool body_closed = true, sup_closed = true;
+  uint8_t *votes[2] = {nullptr, nullptr};
+  GridInfo *info = nullptr;
   cudaError_t e = cudaMalloc(&g->flags, cells * 4);
   float *d_sup = nullptr;
+  if (e == cudaSuccess) e = tmp_alloc(&info, sizeof(GridInfo), s);
   if (e == cudaSuccess) e = tmp_alloc(&d_mesh, (body_triangles ? body_triangles : 1) * 36, s);
   if (e == cudaSuccess) e = tmp_alloc(&d_sup, (support_triangles ? support_triangles : 1) * 36, s);
   if (e != cudaSuccess) rc = cuda_status(e, "pw_voxelize");
   if (rc == PW_OK) {
-    cudaMemsetAsync(g->flags, 0, cells * 4, s);
+    cudaMemsetAsync(info, 0, sizeof(GridInfo), s);
     if (body_triangles) cudaMemcpyAsync(d_mesh, body, (size_t)body_triangles * 36, cudaMemcpyHostToDevice, s);
-    rc = vote_mesh(d_mesh, body_triangles, nx, ny, nz, g->flags, pw::SOLID, &body_closed, s);
+    rc = vote_mesh(d_mesh, body_triangles, nx, ny, nz, 0, info, &votes[0], s);
   }
   if (rc == PW_OK && supports) {
     if (support_triangles) cudaMemcpyAsync(d_sup, supports, (size_t)support_triangles * 36, cudaMemcpyHostToDevice, s);
-    rc = vote_mesh(d_sup, support_triangles, nx, ny, nz, g->flags, pw::SUPPORT, &sup_closed, s);
+    rc = vote_mesh(d_sup, support_triangles, nx, ny, nz, 1, info, &votes[1], s);
   }
-  if (rc == PW_OK) {
-    boundary_kernel<<<nblk(cells), 256, 0, s>>>(g->flags, nx, ny, nz, floor_on);
-    rc = finish_grid(g, floor_on, body_closed, sup_closed, s);
-  }
+  if (rc == PW_OK) rc = finish_grid(g, votes[0], votes[1], floor_on, info, s);
   if (rc == PW_OK && link_fractions && g->nfrac)
     rc = measure_links(g, d_mesh, body_triangles, d_sup, support_triangles, supports != nullptr, floor_on, s);
   tmp_free(d_mesh, s);
   tmp_free(d_sup, s);
-  cudaStreamSynchronize(s);
+  tmp_free(votes[0], s);
+  tmp_free(votes[1], s);
+  tmp_free(info, s);
+  e = cudaStreamSynchronize(s);
+  if (rc == PW_OK && e != cudaSuccess) rc = cuda_status(e, "pw_voxelize");
   cudaStreamDestroy(s);
   if (rc != PW_OK) { delete g; return rc; }
   *out = g;
