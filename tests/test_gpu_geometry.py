@@ -97,3 +97,21 @@ def test_voxelizer_rejects_non_finite_body(value, at):
     bad[at] = value
     with pytest.raises(RangeError):
         voxelize(bad, None, (32, 32, 32), False)
+
+
+# measured fractions: bins of many triangles (several queue flushes a link), of few,
+# a body across the periodic y seam, one without supports' triangles
+@pytest.mark.parametrize("name,make,layout,floor", [
+    ("dense", lambda: (meshes.icosphere((15.3, 14.1, 11.2), 3.3, 4), None), (37, 29, 23), False),
+    ("coarse", lambda: (box([3.2, 4.7, 2.9], [30.1, 25.3, 19.8]), None), (37, 29, 23), True),
+    ("seam", lambda: (meshes.icosphere((15.3, 0.4, 11.2), 4.6, 3), None), (37, 29, 23), False),
+    ("supports", lambda: (meshes.icosphere((15.3, 14.1, 11.2), 4.6, 3), box([13, 12, 0.6], [17, 16, 8.2])),
+     (37, 29, 23), True),
+    ("no support triangles", lambda: (meshes.icosphere((15.3, 14.1, 11.2), 4.6, 2),
+                                      meshes.Mesh(np.zeros(0, np.float32), 0)), (37, 29, 23), False),
+])
+def test_link_fraction_groups(name, make, layout, floor):
+    body, supports = make()
+    g, r = _both(body, supports, layout, floor, True)
+    assert np.array_equal(g.geometry, r.geometry)
+    assert g.missed_links == r.missed_links
