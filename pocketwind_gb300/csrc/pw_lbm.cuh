@@ -1445,9 +1445,11 @@ __global__ void __launch_bounds__(NTHREADS, 8) aa_step_edges(StepParams p, const
 #endif
 
 // ---------------------------------------------------------------- init (layout E)
-// init.wgsl:1-8 into the even layout, after the array was cleared: equilibrium
-// at u_start in fluid and EQ cells, macros everywhere (walls at rest),
-// both outlet planes and both force partials of the start state.
+// init.wgsl:1-8 into the even layout: equilibrium at u_start in fluid and EQ
+// cells, zeros in walls (whose slots the neighbours' bounce-back reads before
+// it first writes them), macros everywhere (walls at rest), both outlet planes
+// and both force partials of the start state.  Every slot of every cell is
+// written, so no pass clears the array first.
 template <int ST>
 __device__ __forceinline__ void init_cell(const StepParams &p, uint32_t x, uint32_t y, uint32_t z, float4 *plane_b,
                                           double &fx, double &fy, double &fz, bool &any) {
@@ -1460,9 +1462,12 @@ __device__ __forceinline__ void init_cell(const StepParams &p, uint32_t x, uint3
   const Nbr b = make_nbr(p, x, y, z);
   const float vx = is_wall_kind(kind) ? 0.0f : p.u_in;
   T code[19];
+  if (is_wall_kind(kind)) {
 #pragma unroll
-  for (int j = 0; j < 19; j++) code[j] = S::encode(geq_ref(j, 0.0f, vx, 0.f, 0.f), (uint32_t)j, n);
-  if (!is_wall_kind(kind)) {
+    for (int j = 0; j < 19; j++) f[(pidx)j * p.stride + n] = T(0.0f);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 19; j++) code[j] = S::encode(geq_ref(j, 0.0f, vx, 0.f, 0.f), (uint32_t)j, n);
 #pragma unroll
     for (int j = 0; j < 19; j++) f[(pidx)opp_of(j) * p.stride + n] = code[j];
     if (kind == FLUID && (flag >> 3)) {
