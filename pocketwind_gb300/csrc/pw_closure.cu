@@ -44,9 +44,21 @@ using namespace pwhost;
 using pw::StepParams;
 using namespace pwcl;
 
-namespace {
+namespace pwclosure_host {
+// Multiprocessors of the current device, cached per device (1 when unknown).
+static int sm_count() {
+  static int sms[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); dev = 0; }
+  if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    sms[dev] = 1;
+  }
+  return std::max(sms[dev], 1);
+}
+}  // namespace pwclosure_host
 
-constexpr int kTrainThreads = 128;
+namespace {
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -865,119 +877,282 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-// One block of kTrainThreads samples: forward with the network's rounding,
-// squared error against the target, backward (the bf16 roundings pass
-// gradients through unchanged; tanh' = 1 - h^2 of the rounded activation),
-// and the block's parameter-gradient sums and loss sum in partial[block].
+// Forward with the network's rounding, squared error against the target, backward
+// (the bf16 roundings pass gradients through unchanged; tanh' = 1 - h^2 of the
+// rounded activation), and the block's parameter-gradient sums and loss sum in
+// partial[block].
 // sample index: explicit list `idx` when given, else mix64(seed + step * 2^32 + i) mod n.
-__global__ void __launch_bounds__(kTrainThreads) train_block(const float *w, const float *X, const float *Y, uint64_t n,
-                                                             uint32_t batch, uint64_t seed, const uint32_t *step,
-                                                             const uint32_t *idx, float *partial) {
-  extern __shared__ float sm[];
-  float *wr = sm;                                     // kParams rounded weights (biases kept)
-  float *xs = wr + kParams + 3;                       // [kTrainThreads][kIn]
-  float *h1s = xs + kTrainThreads * kIn;              // [kTrainThreads][32]
-  float *d1s = h1s + kTrainThreads * kHidden;
-  float *h2s = d1s + kTrainThreads * kHidden;
-  float *d2s = h2s + kTrainThreads * kHidden;
-  float *d3s = d2s + kTrainThreads * kHidden;         // [kTrainThreads]
-  float *ls = d3s + kTrainThreads;                    // [kTrainThreads]
-  const uint32_t tid = threadIdx.x;
-  for (int k = tid; k < kParams; k += kTrainThreads) {
-    const bool bias = (k >= kB1 && k < kW2) || (k >= kB2 && k < kW3) || k == kB3;
-    wr[k] = bias ? w[k] : bf16_round(w[k]);
+//
+// One block of 16 warps an SM.  A warp takes 32 samples at a time, one a lane, and
+// needs no block barrier until its last: weights are broadcast from shared memory
+// four at a time, a lane's activations go to its row of the warp's own buffers
+// (36 words a row: rows and columns both free of bank conflicts as 16-byte pieces),
+// and the gradients are products over the 32 rows with an 8 x 4 tile of dW2 and a
+// row of dW1 in each lane's registers, kept there over all of the warp's samples.
+// It is bound by the binary32 multiply-adds (3,700 a sample, 4 warps a scheduler).
+// 65,536 samples: 26 us; 145 us with a sample a thread, rows of 32 words (every
+// column access 32 ways in conflict) and a thread a parameter for the sums.
+constexpr int kTrainWarps = 16, kTrainThreads = 32 * kTrainWarps;
+constexpr int kRow = 36, kXRow = 12;
+struct TrainWarp {
+  float a[32 * kRow];   // hidden layer 2 (h2, then d2), then d1; at the end the warp's sums
+  float b[32 * kRow];   // hidden layer 1
+  float x[32 * kXRow];  // inputs, 9..11 zero
+};
+struct TrainShared {
+  float w1[kHidden * kXRow], w2[kHidden * kHidden], w3[kHidden], b1[kHidden], b2[kHidden];
+  TrainWarp warp[kTrainWarps];
+};
+static_assert(2 * 32 * kRow >= kParams + 1, "a warp's sums fit its row buffers");
+
+__global__ void __launch_bounds__(kTrainThreads, 1) train_block(const float *w, const float *X, const float *Y,
+                                                               uint64_t n, uint32_t batch, uint64_t seed,
+                                                               const uint32_t *step, const uint32_t *idx,
+                                                               float *partial) {
+  extern __shared__ __align__(16) unsigned char train_smem_raw[];
+  TrainShared &sh = *reinterpret_cast<TrainShared *>(train_smem_raw);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wib = tid >> 5;
+  for (int k = tid; k < kHidden * kXRow; k += kTrainThreads)
+    sh.w1[k] = k % kXRow < kIn ? bf16_round(w[kW1 + k / kXRow * kIn + k % kXRow]) : 0.0f;
+  for (int k = tid; k < kHidden * kHidden; k += kTrainThreads) sh.w2[k] = bf16_round(w[kW2 + k]);
+  if (tid < kHidden) {
+    sh.w3[tid] = bf16_round(w[kW3 + tid]);
+    sh.b1[tid] = w[kB1 + tid];
+    sh.b2[tid] = w[kB2 + tid];
+  }
+  const float b3 = w[kB3];
+  __syncthreads();
+  TrainWarp &my = sh.warp[wib];
+  float *arow = my.a + lane * kRow, *brow = my.b + lane * kRow, *xrow = my.x + lane * kXRow;
+  const float4 *w1v = reinterpret_cast<const float4 *>(sh.w1), *w2v = reinterpret_cast<const float4 *>(sh.w2);
+  const float4 *w3v = reinterpret_cast<const float4 *>(sh.w3);
+  const uint32_t groups = (batch + 31u) / 32u;  // group g: block g mod grid, its warp g / grid mod 16
+  const uint32_t j0 = (lane >> 3) * 8u, k0 = (lane & 7u) * 4u;  // this lane's tile of dW2
+  float g2[8][4], g1[kIn], gb1 = 0.0f, gb2 = 0.0f, g3 = 0.0f, gb3 = 0.0f, loss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) g2[j][k] = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kIn; k++) g1[k] = 0.0f;
+  for (uint32_t g = blockIdx.x + gridDim.x * wib; g < groups; g += gridDim.x * kTrainWarps) {
+    const uint32_t i = g * 32u + lane;
+    const bool live = i < batch;
+    uint64_t s = 0;
+    if (live) s = idx ? idx[i] : mix64(seed + ((uint64_t)*step << 32) + i) % n;
+    const float target = live ? Y[s] : 0.0f;
+    float x[kXRow];
+#pragma unroll
+    for (int k = 0; k < kXRow; k++) x[k] = live && k < kIn ? bf16_round(X[s * kIn + k]) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kXRow; k += 4)
+      *reinterpret_cast<float4 *>(xrow + k) = make_float4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+    // layer 1, four units at a time
+#pragma unroll 1
+    for (int j = 0; j < kHidden; j += 4) {
+      float h[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float4 wa = w1v[3 * (j + q)], wb = w1v[3 * (j + q) + 1];
+        float acc = fmaf(wa.x, x[0], 0.0f);
+        acc = fmaf(wa.y, x[1], acc);
+        acc = fmaf(wa.z, x[2], acc);
+        acc = fmaf(wa.w, x[3], acc);
+        acc = fmaf(wb.x, x[4], acc);
+        acc = fmaf(wb.y, x[5], acc);
+        acc = fmaf(wb.z, x[6], acc);
+        acc = fmaf(wb.w, x[7], acc);
+        acc = fmaf(sh.w1[kXRow * (j + q) + 8], x[8], acc);
+        h[q] = bf16_round(tanh_fast(acc + sh.b1[j + q]));
+      }
+      *reinterpret_cast<float4 *>(brow + j) = make_float4(h[0], h[1], h[2], h[3]);
+    }
+    float out = 0.0f;
+    {
+      float h1[kHidden];
+#pragma unroll
+      for (int k = 0; k < kHidden; k += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(brow + k);
+        h1[k] = v.x; h1[k + 1] = v.y; h1[k + 2] = v.z; h1[k + 3] = v.w;
+      }
+#pragma unroll 1
+      for (int j = 0; j < kHidden; j += 4) {
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < kHidden; k += 4) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const float4 v = w2v[(j + q) * (kHidden / 4) + k / 4];
+            acc[q] = fmaf(v.x, h1[k], acc[q]);
+            acc[q] = fmaf(v.y, h1[k + 1], acc[q]);
+            acc[q] = fmaf(v.z, h1[k + 2], acc[q]);
+            acc[q] = fmaf(v.w, h1[k + 3], acc[q]);
+          }
+        }
+        const float4 w3 = w3v[j / 4];
+        float4 h;
+        h.x = bf16_round(tanh_fast(acc[0] + sh.b2[j]));
+        h.y = bf16_round(tanh_fast(acc[1] + sh.b2[j + 1]));
+        h.z = bf16_round(tanh_fast(acc[2] + sh.b2[j + 2]));
+        h.w = bf16_round(tanh_fast(acc[3] + sh.b2[j + 3]));
+        out = fmaf(w3.x, h.x, out);
+        out = fmaf(w3.y, h.y, out);
+        out = fmaf(w3.z, h.z, out);
+        out = fmaf(w3.w, h.w, out);
+        *reinterpret_cast<float4 *>(arow + j) = h;
+      }
+    }
+    out += b3;
+    const float err = live ? out - target : 0.0f;
+    const float d3 = live ? 2.0f * err / (float)batch : 0.0f;
+    loss += err * err;
+    gb3 += d3;
+    __syncwarp();
+    // dW3: lane j sums d3 h2[j] over the warp's samples
+#pragma unroll 8
+    for (int r = 0; r < 32; r++) g3 = fmaf(__shfl_sync(0xffffffffu, d3, r), my.a[r * kRow + lane], g3);
+    __syncwarp();
+    // d2 over h2, and d1 = (W2^T d2) (1 - h1^2) in registers
+    float d1[kHidden];
+#pragma unroll
+    for (int k = 0; k < kHidden; k++) d1[k] = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < kHidden; j += 4) {
+      const float4 h = *reinterpret_cast<const float4 *>(arow + j), w3 = w3v[j / 4];
+      float d2[4];
+      d2[0] = d3 * w3.x * (1.0f - h.x * h.x);
+      d2[1] = d3 * w3.y * (1.0f - h.y * h.y);
+      d2[2] = d3 * w3.z * (1.0f - h.z * h.z);
+      d2[3] = d3 * w3.w * (1.0f - h.w * h.w);
+      *reinterpret_cast<float4 *>(arow + j) = make_float4(d2[0], d2[1], d2[2], d2[3]);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+#pragma unroll
+        for (int k = 0; k < kHidden; k += 4) {
+          const float4 v = w2v[(j + q) * (kHidden / 4) + k / 4];
+          d1[k] = fmaf(d2[q], v.x, d1[k]);
+          d1[k + 1] = fmaf(d2[q], v.y, d1[k + 1]);
+          d1[k + 2] = fmaf(d2[q], v.z, d1[k + 2]);
+          d1[k + 3] = fmaf(d2[q], v.w, d1[k + 3]);
+        }
+      }
+    }
+    __syncwarp();
+    // dW2 over the 32 rows of d2 and h1; db2 with it
+#pragma unroll 4
+    for (int r = 0; r < 32; r++) {
+      const float4 da = *reinterpret_cast<const float4 *>(my.a + r * kRow + j0);
+      const float4 db = *reinterpret_cast<const float4 *>(my.a + r * kRow + j0 + 4);
+      const float4 h = *reinterpret_cast<const float4 *>(my.b + r * kRow + k0);
+      const float d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        g2[j][0] = fmaf(d[j], h.x, g2[j][0]);
+        g2[j][1] = fmaf(d[j], h.y, g2[j][1]);
+        g2[j][2] = fmaf(d[j], h.z, g2[j][2]);
+        g2[j][3] = fmaf(d[j], h.w, g2[j][3]);
+      }
+      gb2 += my.a[r * kRow + lane];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kHidden; k += 4) {
+      const float4 h = *reinterpret_cast<const float4 *>(brow + k);
+      *reinterpret_cast<float4 *>(arow + k) =
+          make_float4(d1[k] * (1.0f - h.x * h.x), d1[k + 1] * (1.0f - h.y * h.y), d1[k + 2] * (1.0f - h.z * h.z),
+                      d1[k + 3] * (1.0f - h.w * h.w));
+    }
+    __syncwarp();
+    // dW1: lane j over the rows of d1 and x; db1 with it
+#pragma unroll 4
+    for (int r = 0; r < 32; r++) {
+      const float d = my.a[r * kRow + lane];
+      const float4 xa = *reinterpret_cast<const float4 *>(my.x + r * kXRow);
+      const float4 xb = *reinterpret_cast<const float4 *>(my.x + r * kXRow + 4);
+      const float xc = my.x[r * kXRow + 8];
+      g1[0] = fmaf(d, xa.x, g1[0]); g1[1] = fmaf(d, xa.y, g1[1]); g1[2] = fmaf(d, xa.z, g1[2]);
+      g1[3] = fmaf(d, xa.w, g1[3]); g1[4] = fmaf(d, xb.x, g1[4]); g1[5] = fmaf(d, xb.y, g1[5]);
+      g1[6] = fmaf(d, xb.z, g1[6]); g1[7] = fmaf(d, xb.w, g1[7]); g1[8] = fmaf(d, xc, g1[8]);
+      gb1 += d;
+    }
+    __syncwarp();  // the buffers are free again
+  }
+  // the warp's sums into its own buffers, then over the block's warps in order
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    loss += __shfl_down_sync(0xffffffffu, loss, o);
+    gb3 += __shfl_down_sync(0xffffffffu, gb3, o);
+  }
+  float *sum = reinterpret_cast<float *>(&my);  // a and b
+#pragma unroll
+  for (int k = 0; k < kIn; k++) sum[kW1 + lane * kIn + k] = g1[k];
+  sum[kB1 + lane] = gb1;
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+    *reinterpret_cast<float4 *>(sum + kW2 + (j0 + j) * kHidden + k0) =
+        make_float4(g2[j][0], g2[j][1], g2[j][2], g2[j][3]);
+  sum[kB2 + lane] = gb2;
+  sum[kW3 + lane] = g3;
+  if (lane == 0) {
+    sum[kB3] = gb3;
+    sum[kParams] = loss;
   }
   __syncthreads();
-  const uint32_t i = blockIdx.x * kTrainThreads + tid;
-  const bool live = i < batch;
-  uint64_t s = 0;
-  if (live) s = idx ? idx[i] : mix64(seed + ((uint64_t)*step << 32) + i) % n;
-  float x[kIn], h1[kHidden];
-#pragma unroll
-  for (int k = 0; k < kIn; k++) x[k] = live ? bf16_round(X[s * kIn + k]) : 0.0f;
-  for (int j = 0; j < kHidden; j++) {
-    float a = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kIn; k++) a = fmaf(wr[kW1 + j * kIn + k], x[k], a);
-    h1[j] = bf16_round(tanh_fast(a + wr[kB1 + j]));
-  }
-  float out = 0.0f;
-  for (int j = 0; j < kHidden; j++) {
-    float a = 0.0f;
-    for (int k = 0; k < kHidden; k++) a = fmaf(wr[kW2 + j * kHidden + k], h1[k], a);
-    const float h2 = bf16_round(tanh_fast(a + wr[kB2 + j]));
-    h2s[tid * kHidden + j] = h2;
-    out = fmaf(wr[kW3 + j], h2, out);
-  }
-  out += wr[kB3];
-  const float err = live ? out - Y[s] : 0.0f;
-  const float d3 = live ? 2.0f * err / (float)batch : 0.0f;
-  ls[tid] = err * err;
-  d3s[tid] = d3;
-  for (int j = 0; j < kHidden; j++) {
-    const float h2 = h2s[tid * kHidden + j];
-    d2s[tid * kHidden + j] = d3 * wr[kW3 + j] * (1.0f - h2 * h2);
-  }
-  for (int k = 0; k < kHidden; k++) {
-    float a = 0.0f;
-    for (int j = 0; j < kHidden; j++) a = fmaf(d2s[tid * kHidden + j], wr[kW2 + j * kHidden + k], a);
-    d1s[tid * kHidden + k] = a * (1.0f - h1[k] * h1[k]);
-    h1s[tid * kHidden + k] = h1[k];
-  }
-#pragma unroll
-  for (int k = 0; k < kIn; k++) xs[tid * kIn + k] = x[k];
-  __syncthreads();
+  // warps past the last group hold zeros: leave them out
+  const uint32_t own = groups > blockIdx.x ? (groups - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+  const uint32_t warps = min(own, (uint32_t)kTrainWarps);
   float *out_p = partial + (size_t)blockIdx.x * (kParams + 1);
   for (int q = tid; q < kParams + 1; q += kTrainThreads) {
     float acc = 0.0f;
-    if (q < kB1) {
-      const int j = q / kIn, k = q % kIn;
-      for (int r = 0; r < kTrainThreads; r++) acc = fmaf(d1s[r * kHidden + j], xs[r * kIn + k], acc);
-    } else if (q < kW2) {
-      for (int r = 0; r < kTrainThreads; r++) acc += d1s[r * kHidden + (q - kB1)];
-    } else if (q < kB2) {
-      const int j = (q - kW2) / kHidden, k = (q - kW2) % kHidden;
-      for (int r = 0; r < kTrainThreads; r++) acc = fmaf(d2s[r * kHidden + j], h1s[r * kHidden + k], acc);
-    } else if (q < kW3) {
-      for (int r = 0; r < kTrainThreads; r++) acc += d2s[r * kHidden + (q - kB2)];
-    } else if (q < kB3) {
-      for (int r = 0; r < kTrainThreads; r++) acc = fmaf(d3s[r], h2s[r * kHidden + (q - kW3)], acc);
-    } else if (q == kB3) {
-      for (int r = 0; r < kTrainThreads; r++) acc += d3s[r];
-    } else {
-      for (int r = 0; r < kTrainThreads; r++) acc += ls[r];
-    }
+    for (uint32_t v = 0; v < warps; v++) acc += reinterpret_cast<const float *>(&sh.warp[v])[q];
     out_p[q] = acc;
   }
 }
 
-// Fixed-order sums of the block partials: grad[q], q < kParams; grad[kParams] = loss sum.
-__global__ void train_reduce(const float *partial, uint32_t blocks, float *grad) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q > (uint32_t)kParams) return;
+// The block partials' sums, grad[q] for q < kParams and grad[kParams] the loss sum, in
+// an order that the block count alone sets: 16 threads a parameter, each every 16th
+// block, then those 16 in order.  With w also Adam (beta1 0.9, beta2 0.999, eps 1e-8)
+// on the binary32 master weights, the batch loss, and, by the last block to come
+// here, the step counter (the other blocks have read it by then).  6.4 us with 152
+// partials; six blocks of a thread a parameter over 512 partials, and Adam in a
+// launch of its own, took 28 us.
+constexpr int kReduceParams = 32, kReduceSplit = 16;
+constexpr int kReduceBlocks = (kParams + 1 + kReduceParams - 1) / kReduceParams;
+__global__ void __launch_bounds__(kReduceParams * kReduceSplit) train_reduce(const float *partial, uint32_t blocks,
+                                                                            float *grad, float *w, float *m, float *v,
+                                                                            uint32_t *step, uint32_t *ticket, float lr,
+                                                                            uint32_t batch, float *loss) {
+  __shared__ float part[kReduceSplit][kReduceParams];
+  const uint32_t c = threadIdx.x % kReduceParams, r = threadIdx.x / kReduceParams;
+  const uint32_t q = blockIdx.x * kReduceParams + c;
   float acc = 0.0f;
-  for (uint32_t b = 0; b < blocks; b++) acc += partial[(size_t)b * (kParams + 1) + q];
-  grad[q] = acc;
-}
-
-// Adam (beta1 0.9, beta2 0.999, eps 1e-8) on the binary32 master weights; one
-// block, which then advances the step counter and records the batch loss.
-__global__ void train_adam(float *w, float *m, float *v, const float *grad, uint32_t *step, float lr, uint32_t batch,
-                           float *loss) {
-  const uint32_t t = *step + 1;
-  const float c1 = 1.0f - powf(0.9f, (float)t), c2 = 1.0f - powf(0.999f, (float)t);
-  for (int q = threadIdx.x; q < kParams; q += blockDim.x) {
-    const float gq = grad[q];
-    const float mq = 0.9f * m[q] + 0.1f * gq;
-    const float vq = 0.999f * v[q] + 0.001f * gq * gq;
-    m[q] = mq;
-    v[q] = vq;
-    w[q] -= lr * (mq / c1) / (sqrtf(vq / c2) + 1e-8f);
-  }
+  if (q <= (uint32_t)kParams)
+    for (uint32_t b = r; b < blocks; b += kReduceSplit) acc += partial[(size_t)b * (kParams + 1) + q];
+  part[r][c] = acc;
+  const uint32_t t = w ? *step + 1u : 0u;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    *loss = grad[kParams] / (float)batch;
-    *step = t;
+  if (r == 0 && q <= (uint32_t)kParams) {
+    acc = part[0][c];
+#pragma unroll
+    for (int k = 1; k < kReduceSplit; k++) acc += part[k][c];
+    grad[q] = acc;
+    if (w && q < (uint32_t)kParams) {
+      const float c1 = 1.0f - powf(0.9f, (float)t), c2 = 1.0f - powf(0.999f, (float)t);
+      const float mq = 0.9f * m[q] + 0.1f * acc;
+      const float vq = 0.999f * v[q] + 0.001f * acc * acc;
+      m[q] = mq;
+      v[q] = vq;
+      w[q] -= lr * (mq / c1) / (sqrtf(vq / c2) + 1e-8f);
+    } else if (w) {
+      *loss = acc / (float)batch;
+    }
+  }
+  if (w && threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(ticket, 1u) + 1u == gridDim.x) {
+      *ticket = 0u;
+      *step = t;
+    }
   }
 }
 
@@ -985,7 +1160,7 @@ __global__ void train_adam(float *w, float *m, float *v, const float *grad, uint
 
 struct pw_closure {
   float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *partial = nullptr, *loss = nullptr;
-  uint32_t *frag = nullptr, *step = nullptr;
+  uint32_t *frag = nullptr, *step = nullptr;  // step[0]: steps taken; step[1]: the reducing blocks' ticket
   float *X = nullptr, *Y = nullptr;
   uint64_t n = 0, cap = 0;
   uint32_t partial_blocks = 0;
@@ -994,8 +1169,9 @@ struct pw_closure {
 
 namespace {
 
-size_t train_smem() {
-  return sizeof(float) * (kParams + 3 + kTrainThreads * (kIn + 4 * kHidden + 2));
+// Blocks of a training pass: one an SM, fewer for a batch of fewer groups of 32.
+uint32_t train_blocks(uint32_t batch) {
+  return std::min((batch + 31u) / 32u, (uint32_t)pwclosure_host::sm_count());
 }
 
 int ensure_partials(pw_closure *c, uint32_t blocks) {
@@ -1009,7 +1185,7 @@ int ensure_partials(pw_closure *c, uint32_t blocks) {
 }
 
 int refresh_fragments(pw_closure *c) {
-  build_fragments<<<1, 32, 0, c->stream>>>(c->w, c->frag);
+  build_fragments<<<1, 1024, 0, c->stream>>>(c->w, c->frag);
   PW_TRY(cudaGetLastError());
   return PW_OK;
 }
@@ -1017,18 +1193,6 @@ int refresh_fragments(pw_closure *c) {
 }  // namespace
 
 namespace pwclosure_host {
-// Multiprocessors of the current device, cached per device (1 when unknown).
-static int sm_count() {
-  static int sms[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); dev = 0; }
-  if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    sms[dev] = 1;
-  }
-  return std::max(sms[dev], 1);
-}
-
 // The closure step for a domain with an attached closure (pw_domain.cu).
 void launch_closure_step(const StepParams &p, int storage, int op, bool odd, dim3 grid, const uint32_t *frag,
                          const uint8_t *wall, cudaStream_t s) {
@@ -1129,9 +1293,9 @@ int pw_closure_create(uint64_t seed, pw_closure **out) {
   if (e == cudaSuccess) e = cudaMalloc(&c->m, kParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&c->v, kParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&c->grad, (kParams + 1) * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&c->loss, sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&c->loss, 2 * sizeof(float));  // the latest step's, a call's first
   if (e == cudaSuccess) e = cudaMalloc(&c->frag, 32 * kFragWords * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&c->step, sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(&c->step, 2 * sizeof(uint32_t));
   if (e != cudaSuccess) {
     int rc = cuda_status(e, "pw_closure_create");
     pw_closure_destroy(c);
@@ -1155,7 +1319,7 @@ int pw_closure_create(uint64_t seed, pw_closure **out) {
   e = cudaMemcpy(c->w, w.data(), kParams * sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(c->m, 0, kParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(c->v, 0, kParams * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemset(c->step, 0, sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemset(c->step, 0, 2 * sizeof(uint32_t));
   if (e != cudaSuccess) {
     int rc = cuda_status(e, "pw_closure_create");
     pw_closure_destroy(c);
@@ -1231,10 +1395,10 @@ int pw_closure_gradients(pw_closure *c, const float *x, const float *y, uint32_t
   if (!c || !x || !y || !grad || count == 0) { set_error("NULL argument or no samples"); return PW_ERR_INVALID; }
   float *dx = nullptr, *dy = nullptr;
   uint32_t *idx = nullptr;
-  const uint32_t blocks = (count + kTrainThreads - 1) / kTrainThreads;
+  const uint32_t blocks = train_blocks(count);
   int rc = ensure_partials(c, blocks);
   if (rc != PW_OK) return rc;
-  PW_TRY(cudaFuncSetAttribute(train_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
+  PW_TRY(cudaFuncSetAttribute(train_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainShared)));
   cudaError_t e = cudaMalloc(&dx, (size_t)count * kIn * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&dy, (size_t)count * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&idx, (size_t)count * sizeof(uint32_t));
@@ -1244,9 +1408,10 @@ int pw_closure_gradients(pw_closure *c, const float *x, const float *y, uint32_t
   if (e == cudaSuccess) e = cudaMemcpyAsync(dy, y, (size_t)count * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(idx, seq.data(), (size_t)count * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
-    train_block<<<blocks, kTrainThreads, train_smem(), c->stream>>>(c->w, dx, dy, count, count, 0, c->step, idx,
-                                                                    c->partial);
-    train_reduce<<<(kParams + 1 + 255) / 256, 256, 0, c->stream>>>(c->partial, blocks, c->grad);
+    train_block<<<blocks, kTrainThreads, sizeof(TrainShared), c->stream>>>(c->w, dx, dy, count, count, 0, c->step, idx,
+                                                                           c->partial);
+    train_reduce<<<kReduceBlocks, kReduceParams * kReduceSplit, 0, c->stream>>>(
+        c->partial, blocks, c->grad, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0f, count, nullptr);
     e = cudaGetLastError();
   }
   std::vector<float> h(kParams + 1);
@@ -1369,19 +1534,20 @@ int pw_closure_train(pw_closure *c, uint32_t steps, uint32_t batch, float lr, ui
                      float *loss_last) {
   if (!c || steps == 0 || batch == 0 || !(lr > 0.0f)) { set_error("Training needs steps, a batch and a positive rate."); return PW_ERR_INVALID; }
   if (c->n == 0) { set_error("The closure dataset is empty."); return PW_ERR_INVALID; }
-  const uint32_t blocks = (batch + kTrainThreads - 1) / kTrainThreads;
+  const uint32_t blocks = train_blocks(batch);
   int rc = ensure_partials(c, blocks);
   if (rc != PW_OK) return rc;
-  PW_TRY(cudaFuncSetAttribute(train_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
+  PW_TRY(cudaFuncSetAttribute(train_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainShared)));
   auto one = [&](cudaStream_t s) {
-    train_block<<<blocks, kTrainThreads, train_smem(), s>>>(c->w, c->X, c->Y, c->n, batch, seed, c->step, nullptr,
-                                                            c->partial);
-    train_reduce<<<(kParams + 1 + 255) / 256, 256, 0, s>>>(c->partial, blocks, c->grad);
-    train_adam<<<1, 1024, 0, s>>>(c->w, c->m, c->v, c->grad, c->step, lr, batch, c->loss);
+    train_block<<<blocks, kTrainThreads, sizeof(TrainShared), s>>>(c->w, c->X, c->Y, c->n, batch, seed, c->step,
+                                                                   nullptr, c->partial);
+    train_reduce<<<kReduceBlocks, kReduceParams * kReduceSplit, 0, s>>>(c->partial, blocks, c->grad, c->w, c->m, c->v,
+                                                                        c->step, c->step + 1, lr, batch, c->loss);
   };
   one(c->stream);
   PW_TRY(cudaGetLastError());
-  if (loss_first) PW_TRY(cudaMemcpyAsync(loss_first, c->loss, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+  // kept on the device until the end: a copy to the host here would hold back the launches
+  PW_TRY(cudaMemcpyAsync(c->loss + 1, c->loss, sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
   // the rest as replays of a captured 100-step graph
   uint32_t done = 1;
   const uint32_t chunk = 100;
@@ -1407,10 +1573,13 @@ int pw_closure_train(pw_closure *c, uint32_t steps, uint32_t batch, float lr, ui
   if (exec) cudaGraphExecDestroy(exec);
   for (; done < steps; done++) one(c->stream);
   PW_TRY(cudaGetLastError());
-  if (loss_last) PW_TRY(cudaMemcpyAsync(loss_last, c->loss, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   rc = refresh_fragments(c);
   if (rc != PW_OK) return rc;
+  float losses[2];
+  PW_TRY(cudaMemcpyAsync(losses, c->loss, sizeof losses, cudaMemcpyDeviceToHost, c->stream));
   PW_TRY(cudaStreamSynchronize(c->stream));
+  if (loss_last) *loss_last = losses[0];
+  if (loss_first) *loss_first = losses[1];
   return PW_OK;
 }
 

@@ -108,6 +108,26 @@ def test_gradients_match_oracle():
 
 
 @pytest_gpu
+@pytest.mark.parametrize("count", [1, 31, 33, 4863, 4865, 77825])
+def test_gradients_match_oracle_at_group_edges(count):
+    """Counts around a warp's 32 samples, a block's first warp (152 blocks) and the
+    whole grid (a warp's second group).  The last sample's target outweighs all
+    others, so leaving it out shows; the tolerance is that of the network's
+    rounding (one bfloat16 step of an activation is 0.4%)."""
+    w = _rand_params(6, 0.3)
+    c = _closure(w)
+    r = np.random.default_rng(count)
+    x = r.uniform(-1, 1, (count, OC.N_IN)).astype(np.float32)
+    y = r.uniform(-1, 1, count).astype(np.float32)
+    y[-1] = 30.0 * np.sqrt(count)
+    loss, g = c.gradients(x, y)
+    rl, rg = OC.gradients(w, x, y)
+    assert loss == pytest.approx(rl, rel=2e-2)
+    assert np.linalg.norm(g - rg) / np.linalg.norm(rg) < 2e-2
+    c.destroy()
+
+
+@pytest_gpu
 def test_one_adam_step_matches_oracle():
     """A dataset of one repeated sample makes every drawn batch the same, so one
     training step is one Adam step on that sample's gradient."""
