@@ -25,6 +25,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           f"-I{INCLUDE}", "--expt-relaxed-constexpr"]
 UNITS = {
     "pw_kernels_fast.cu": [],
+    "pw_kernels_all.cu": [],
     "pw_kernels_strict.cu": ["-fmad=false"],
     "pw_geometry.cu": ["-fmad=false"],
     "pw_tracers.cu": ["-fmad=false"],

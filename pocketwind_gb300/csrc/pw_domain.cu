@@ -199,6 +199,7 @@ struct pw_domain {
   dim3 grid;
   uint32_t slip = 0;              // free-slip faces (bit 0 y, bit 1 z)
   bool split = false;             // fast build, one cell per thread: plain kernel + edge list
+  bool one_launch = false;        // a split step as one launch
   uint32_t *edges = nullptr;      // edge cells in ascending order
   uint32_t edge_count = 0;
   uint32_t edge_own = 0;          // the list's head that a domain's own step runs (all but its floor cells)
@@ -294,6 +295,8 @@ void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro) {
   else if (d->closure_frag)
     pwclosure_host::launch_closure_step(p, d->desc.storage, d->desc.op, odd, d->grid, d->closure_frag, d->wall_dist,
                                         d->stream);
+  else if (d->one_launch && d->split)
+    pwall::launch_step_all(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->edges, d->edge_own, d->stream);
   else if (d->split)
     pwfast::launch_step_split(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->plain_grid, d->edges,
                               d->edge_own, d->stream, nullptr, &d->side);
@@ -642,6 +645,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   int rc = PW_OK;
   if (!d->tiled && !desc->strict) {
     d->split = true;
+    d->one_launch = pwall::step_all_supported(d->nx, d->ny, d->nz, desc->storage, desc->les, d->slip);
     rc = build_edge_list(d, a);
   }
   if (rc == PW_OK) rc = launch_init(d);
@@ -705,8 +709,14 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
     d->steps++;
     k++;
   }
-  // full-speed steps: graph chunks when the domain is small enough to be launch bound
-  const bool use_graphs = d->cells <= (size_t)8 << 20;
+  // full-speed steps: graph chunks when the domain is small enough to be launch bound.
+  // A step of one launch needs none (its successor is launched while it runs; in a graph
+  // the 128x64x64 FP32 vehicle's step took as long), and a split step of more than a
+  // million cells is faster without (its side kernels lose their head start in a graph:
+  // 192x96x96 FP16 45.9 us a step against 37.9; 128x64x64 24.0 against 28.9).
+  const bool one_launch = d->one_launch && !d->closure_frag;
+  const bool split = d->split && !d->closure_frag;
+  const bool use_graphs = !one_launch && d->cells <= (size_t)(split ? 1 : 8) << 20;
   while (use_graphs && count - k >= (uint64_t)kGraphChunk) {
     int macro_last = write_macro_on_last && (count - k == (uint64_t)kGraphChunk);
     cudaGraphExec_t g = graph_for(d, (int)((d->steps + 1) & 1), macro_last);

@@ -58,6 +58,12 @@ void launch_refresh_edges(const pw::StepParams &p, int odd_layout, int storage, 
                           uint32_t count, cudaStream_t s);
 }
 PW_DECLARE_LAUNCHERS(pwstrict)
+// The same split step in one launch, blocks by role (pw_kernels_all.cu).
+namespace pwall {
+bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int les, uint32_t slip);
+void launch_step_all(const pw::StepParams &p, int storage, int op, int les, bool odd, const uint32_t *list,
+                     uint32_t count, cudaStream_t s);
+}
 
 
 struct pw_closure;

@@ -1291,13 +1291,16 @@ __device__ __forceinline__ void pair_cells(const StepParams &p, uint32_t n, uint
 // on the side stream.  Floor cells link only to FLOOR cells, which add
 // nothing to the drag.
 template <int ST, int OP, bool LES, bool ODD>
-__global__ void __launch_bounds__(NTHREADS, 5) aa_step_floor(StepParams p) {
-  const uint32_t x = blockIdx.x * (2 * BX) + 2u * threadIdx.x;
-  const uint32_t y = 1u + blockIdx.y * BY + threadIdx.y;
+__device__ __forceinline__ void floor_thread(const StepParams &p, uint32_t x, uint32_t y) {
   if (x >= p.nx || y + 2u > p.ny) return;
   const uint32_t n = x + p.nx * (y + p.ny);
   const uint32_t ok = (__ldg(&p.flags[n]) == kFloorFlag ? 1u : 0u) | (__ldg(&p.flags[n + 1]) == kFloorFlag ? 2u : 0u);
   if (ok) pair_cells<ST, OP, LES, ODD, true>(p, n, x, y, 1u, ok, 0u);
+}
+
+template <int ST, int OP, bool LES, bool ODD>
+__global__ void __launch_bounds__(NTHREADS, 5) aa_step_floor(StepParams p) {
+  floor_thread<ST, OP, LES, ODD>(p, blockIdx.x * (2 * BX) + 2u * threadIdx.x, 1u + blockIdx.y * BY + threadIdx.y);
 }
 
 template <int ST, int OP, bool LES, bool ODD>
