@@ -212,6 +212,7 @@ struct StepParams {
   uint32_t *status;        // bit 0: density guard tripped on a macro step
   uint32_t nx, ny, nz;
   uint32_t stride;         // elements between direction planes
+  uint32_t inv_nx;         // floor((2^32 - 1) / nx) + 1: rows of a plane's cells without a division
   float u_in;              // inlet speed of this step
   float nu, cs_term, lambda;
   float tau0, omega_plus, omega_minus;  // binary32 constants of the LES-free operator

@@ -243,6 +243,7 @@ pw::StepParams params_for(const pw_domain *d, uint64_t step, float u_in, int wri
   p.status = d->status_dev;
   p.nx = d->nx; p.ny = d->ny; p.nz = d->nz;
   p.stride = d->stride;
+  p.inv_nx = 0xffffffffu / d->nx + 1u;
   p.u_in = u_in;
   p.nu = d->nu; p.cs_term = d->cs_term; p.lambda = d->lambda;
   p.tau0 = d->tau0; p.omega_plus = d->om_p; p.omega_minus = d->om_m;

@@ -1322,6 +1322,143 @@ __device__ __forceinline__ void pair_thread(const StepParams &p, uint32_t x, uin
   if (ok) pair_cells<ST, OP, LES, ODD>(p, n, x, y, z, ok, eq);
 }
 
+// ---------------------------------------------------------------- 16-bit pairs, nx odd
+// With nx odd the rows do not start on a word, so the pairs run over a plane's cells in
+// their order: cells n and n + 1 with n even, which may be the last cell of one row and
+// the first of the next.  Even steps touch own slots only: every direction is a word, as
+// for even nx.  On odd steps direction i sits off the word grid when its element offset
+// c_x + nx c_y + nx ny c_z is odd: 12 directions for ny even, 6 for ny odd (one 16-bit
+// access a cell for those); no lane idles at a row's end.  It is bound by its issue slots
+// and memory latency, as the pairs for even nx.  FP16 at 203x101x67: 24 us a step (65% of
+// the copy bandwidth); cells x and x + 32 of a run, 76 16-bit accesses a lane and a sixth
+// of the lanes idle, took 33.
+template <bool ODD, bool NY_ODD>
+__host__ __device__ constexpr bool linear_shifted(int i) {
+  return ODD && ((cx_of(i) + cy_of(i) + (NY_ODD ? cz_of(i) : 0)) & 1) != 0;
+}
+
+// Cell m of a plane as its row and place: m / nx by inv_nx = floor((2^32 - 1) / nx) + 1
+// (too large by at most one).
+__device__ __forceinline__ void plane_cell(const StepParams &p, uint32_t m, uint32_t &x, uint32_t &y) {
+  y = __umulhi(m, p.inv_nx);
+  uint32_t first = y * p.nx;
+  if (first > m) { y--; first -= p.nx; }
+  x = m - first;
+}
+
+// Cells n and n + 1 (n even) of plane z, m their place in the plane (m = -1: the pair
+// begins in the plane before).
+template <int ST, int OP, bool LES, bool ODD, bool NY_ODD>
+__device__ __forceinline__ void linear_thread(const StepParams &p, int32_t m, uint32_t z) {
+  using S = Store<ST>;
+  const uint32_t plane = p.nx * p.ny;
+  if (m >= (int32_t)plane) return;
+  const uint32_t n = plane * z + (uint32_t)m;
+  const uint32_t word = __ldg(&p.special[n >> 5]);
+  // what the update and the stores need of the two cells, a bit a lane each in one
+  // register: stored here (bits 0, 1), EQ (2, 3), EQ at x = 0 (4, 5), EQ at x = nx - 1
+  // (6, 7), at x = nx - 2 (8, 9)
+  uint32_t st = 0u;
+#pragma unroll
+  for (uint32_t k = 0; k < 2u; k++) {
+    const uint32_t mk = (uint32_t)m + k;
+    if (mk >= plane) continue;  // the plane before (m = -1) or after
+    uint32_t x, y;
+    plane_cell(p, mk, x, y);
+    if (ODD && (y == 0u || y + 1u == p.ny)) continue;  // seam rows
+    uint32_t b = 0u;
+    if (!((word >> ((n + k) & 31u)) & 1u)) {
+      if (is_plain_position(x, p.nx)) b = 1u;
+    } else if (__ldg(&p.flags[n + k]) == EQ) {
+      b = 5u | (x == 0u ? 16u : 0u) | (x + 1u == p.nx ? 64u : 0u);
+    }
+    if (b && x + 2u == p.nx) b |= 256u;
+    st |= b << k;
+  }
+  if (!(st & 3u)) return;
+  char *const base = reinterpret_cast<char *>(p.f) + 2 * (size_t)n;
+  float2 g[19];
+#pragma unroll
+  for (int i = 0; i < 19; i++) {
+    const char *a = base + p.ldb[i];
+    if (linear_shifted<ODD, NY_ODD>(i)) g[i] = make_float2(raw_of_bits<ST>(ld_half(a)), raw_of_bits<ST>(ld_half(a + 2)));
+    else g[i] = raw_of_word<ST>(ld_word(a));
+  }
+  float2 eux = f2(p.u_in), euy = f2(0.f), euz = f2(0.f);
+  if (st & 0xc0u) {  // the outlet
+    uint32_t x, y;
+    plane_cell(p, (uint32_t)m + ((st & 0x40u) ? 0u : 1u), x, y);
+    const float4 u = p.plane_in[y + p.ny * z];
+    if (st & 0x40u) { eux.x = u.x; euy.x = u.y; euz.x = u.z; }
+    else { eux.y = u.x; euy.y = u.y; euz.y = u.z; }
+  }
+  float2 rho, vx, vy, vz;
+  const float2 om =
+      update_fast2<OP, LES>(p, g, rho, vx, vy, vz, S::kScale, S::kInvScale, (st >> 2) & 3u, eux, euy, euz);
+  // a non-finite state is stored as NaN, as the reference's GPUs store it
+  if (!(fabsf(rho.x + om.x) < INFINITY)) {
+#pragma unroll
+    for (int j = 0; j < 19; j++) g[j].x = __uint_as_float(0x7fc00000u);
+  }
+  if (!(fabsf(rho.y + om.y) < INFINITY)) {
+#pragma unroll
+    for (int j = 0; j < 19; j++) g[j].y = __uint_as_float(0x7fc00000u);
+  }
+  const uint32_t nk = n * 0x9e3779b9u, nk2 = nk + 0x9e3779b9u;
+  uint32_t w[19];
+#pragma unroll
+  for (int j = 0; j < 19; j++)
+    w[j] = S::encode_pair(g[j].y, g[j].x, pair_dither<ST>(g[j].y, g[j].x, dither_mul(j), nk2, nk));
+  // odd steps: the EQ cell at x = 0 pushes c_x = -1 to x = nx - 1 and the one at
+  // x = nx - 1 pushes c_x = +1 to x = 0 (periodic in x)
+  if ((st & 3u) == 3u && !(ODD && (st & 0xf0u))) {
+#pragma unroll
+    for (int j = 0; j < 19; j++) {
+      char *a = base + p.stb[j];
+      if (linear_shifted<ODD, NY_ODD>(j)) {
+        st_half(a, w[j] & 0xffffu);
+        st_half(a + 2, w[j] >> 16);
+      } else {
+        st_word(a, w[j]);
+      }
+    }
+  } else {
+    const int back = ODD ? 2 * (int)p.nx : 0;
+#pragma unroll
+    for (int j = 0; j < 19; j++) {
+      char *a = base + p.stb[j];
+      const int wa = cx_of(j) < 0 && (st & 16u) ? back : (cx_of(j) > 0 && (st & 64u) ? -back : 0);
+      const int wb = cx_of(j) < 0 && (st & 32u) ? back : (cx_of(j) > 0 && (st & 128u) ? -back : 0);
+      if (st & 1u) st_half(a + wa, w[j] & 0xffffu);
+      if (st & 2u) st_half(a + 2 + wb, w[j] >> 16);
+    }
+  }
+  // the outlet's upstream cell (x = nx - 2) publishes the velocity of its stored codes
+  // (outlet_velocity_of)
+  if (st & 0x300u) {
+    const bool a = (st & 0x100u) != 0u;
+    float mass = 1.0f, mx = 0.f, my = 0.f, mz = 0.f;
+#pragma unroll
+    for (int j = 0; j < 19; j++) {
+      const float v = raw_of_bits<ST>(a ? w[j] & 0xffffu : w[j] >> 16) * S::kInvScale;
+      mass += v;
+      mx += (float)cx_of(j) * v;
+      my += (float)cy_of(j) * v;
+      mz += (float)cz_of(j) * v;
+    }
+    uint32_t x, y;
+    plane_cell(p, (uint32_t)m + (a ? 0u : 1u), x, y);
+    p.plane_out[y + p.ny * z] = make_float4(mx / mass, my / mass, mz / mass, 0.f);
+  }
+  if (p.write_macro) {
+    const bool bad_a = (st & 5u) == 1u && !(rho.x >= 0.5f && rho.x <= 1.5f);
+    const bool bad_b = (st & 10u) == 2u && !(rho.y >= 0.5f && rho.y <= 1.5f);
+    if (bad_a || bad_b) atomicOr(p.status, 1u);
+    if (st & 1u) p.macros[n] = make_float4(rho.x, vx.x, vy.x, vz.x);
+    if (st & 2u) p.macros[n + 1] = make_float4(rho.y, vx.y, vy.y, vz.y);
+  }
+}
+
 // One warp per 64-cell run of a row: every row on even steps, the rows off the
 // periodic y and z seams on odd steps.  Held to 64 registers (8 blocks per SM):
 // the few spilled words cost less than the lost occupancy (measured 1%).
