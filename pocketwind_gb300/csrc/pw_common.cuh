@@ -217,6 +217,7 @@ struct StepParams {
   float nu, cs_term, lambda;
   float tau0, omega_plus, omega_minus;  // binary32 constants of the LES-free operator
   int write_macro;
+  int clear_status;        // this step clears the guard's flag (one-launch steps; a macro step follows)
   uint32_t slip;           // free-slip faces: bit 0 the y faces, bit 1 the z faces (0: periodic)
   // Plain cells (no periodic wrap in reach): direction i is loaded from element
   // n + ld[i] and stored to element n + st[i] of f, offsets for this step's parity.

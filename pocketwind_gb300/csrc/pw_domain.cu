@@ -143,8 +143,11 @@ __global__ void clear_slip_links_kernel(uint32_t *flags, uint32_t nx, uint32_t n
 }
 
 // Sum both parities' partials: 0.5 * (F(even state) + F(odd state)) (force.wgsl:31-32,
-// reduce.wgsl), binary64, fixed order.
+// reduce.wgsl), binary64, fixed order, straight into the pinned staging slot: a copy
+// behind the kernel cost 5 us of a frame.  The block is launched while the step before
+// it runs and waits for its end.
 __global__ void force_reduce_kernel(const double *a, const double *b, size_t nblocks, double *out) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ double sh[256][3];
   double s0 = 0, s1 = 0, s2 = 0;
   for (size_t k = threadIdx.x; k < nblocks; k += 256) {
@@ -159,8 +162,7 @@ __global__ void force_reduce_kernel(const double *a, const double *b, size_t nbl
       for (int c = 0; c < 3; c++) sh[threadIdx.x][c] += sh[threadIdx.x + st][c];
     __syncthreads();
   }
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; c++) out[c] = 0.5 * sh[0][c];
+  if (threadIdx.x < 3) out[threadIdx.x] = 0.5 * sh[0][threadIdx.x];
 }
 
 enum ForceState { FORCE_IDLE = 0, FORCE_ENCODED = 1 };
@@ -182,8 +184,7 @@ struct pw_domain {
   float wall_c = 0, wall_e = 0;   // Werner-Wengle constants of the floor cells' wall model
   double *partials[2] = {nullptr, nullptr};
   size_t nblocks = 0;
-  double *force_dev = nullptr;
-  double *force_host = nullptr;   // pinned staging slot
+  double *force_host = nullptr;   // pinned staging slot, written by the reduction
   uint32_t *status_dev = nullptr;
   uint32_t *status_host = nullptr;
   double *totals_dev = nullptr;
@@ -277,10 +278,15 @@ pw::StepParams params_for(const pw_domain *d, uint64_t step, float u_in, int wri
   return p;
 }
 
-// Queue step number `step` (1-based) with the given inlet speed.
-void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro) {
+// Queue step number `step` (1-based) with the given inlet speed.  The guard's flag of a
+// macro step starts at zero: a step of one launch before it in the same call clears it
+// (before_macro, then cleared), without a memset between the two.
+void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool before_macro = false,
+                  bool cleared = false) {
   pw::StepParams p = params_for(d, step, u_in, write_macro);
-  if (write_macro) cudaMemsetAsync(d->status_dev, 0, 4, d->stream);
+  const bool one = d->one_launch && d->split && !d->closure_frag;
+  p.clear_status = one && before_macro ? 1 : 0;
+  if (write_macro && !(one && cleared)) cudaMemsetAsync(d->status_dev, 0, 4, d->stream);
   bool odd = (step & 1) != 0;
   if (d->tiled && d->desc.strict)
     pwstrict::launch_step_tile(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->rows_per_tile, d->tile_blocks,
@@ -592,7 +598,6 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   if (d->interp && e == cudaSuccess) e = a.alloc(&d->hist, (grid->nfrac ? grid->nfrac : 1) * d->esize);
   if (e == cudaSuccess) e = a.alloc((void **)&d->partials[0], d->nblocks * 3 * sizeof(double));
   if (e == cudaSuccess) e = a.alloc((void **)&d->partials[1], d->nblocks * 3 * sizeof(double));
-  if (e == cudaSuccess) e = a.alloc((void **)&d->force_dev, 4 * sizeof(double));
   if (e == cudaSuccess) e = a.alloc((void **)&d->status_dev, 16);
   if (e == cudaSuccess) e = a.alloc((void **)&d->totals_dev, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost((void **)&d->force_host, 4 * sizeof(double));
@@ -675,7 +680,7 @@ void pw_domain_destroy(pw_domain *d) {
   drop_graphs(d);
   cudaFree(d->f); cudaFree(d->macros); cudaFree(d->plane[0]); cudaFree(d->plane[1]);
   cudaFree(d->flags); cudaFree(d->special); cudaFree(d->partials[0]); cudaFree(d->partials[1]);
-  cudaFree(d->force_dev); cudaFree(d->status_dev); cudaFree(d->totals_dev); cudaFree(d->scratch);
+  cudaFree(d->status_dev); cudaFree(d->totals_dev); cudaFree(d->scratch);
   cudaFree(d->edges);
   cudaFree(d->wall_dist);
   cudaFree(d->qoff); cudaFree(d->qfrac); cudaFree(d->hist);
@@ -706,7 +711,8 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
   // ramped steps, one launch each with its own inlet speed
   while (k < count && d->desc.ramp_steps > 0 && d->steps < d->desc.ramp_steps) {
     uint64_t step = d->steps + 1;
-    enqueue_step(d, step, ramp_speed(d, step), write_macro_on_last && k == count - 1);
+    enqueue_step(d, step, ramp_speed(d, step), write_macro_on_last && k == count - 1,
+                 write_macro_on_last && k + 2 == count, k > 0);
     d->steps++;
     k++;
   }
@@ -728,7 +734,7 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
   }
   for (; k < count; k++) {
     uint64_t step = d->steps + 1;
-    enqueue_step(d, step, d->u_in, write_macro_on_last && k == count - 1);
+    enqueue_step(d, step, d->u_in, write_macro_on_last && k == count - 1, write_macro_on_last && k + 2 == count, k > 0);
     d->steps++;
   }
   PW_TRY(cudaGetLastError());
@@ -745,8 +751,17 @@ int pw_encode_force(pw_domain *d) {
   if (!alive(d)) return PW_ERR_INVALID;
   if (d->force_state != FORCE_IDLE) return PW_OK;  // occupied slot skips the sample
   if (d->interp) interp_state(d, d->steps, 0);  // the latest state; the last step gave the one before
-  force_reduce_kernel<<<1, 256, 0, d->stream>>>(d->partials[0], d->partials[1], d->nblocks, d->force_dev);
-  PW_TRY(cudaMemcpyAsync(d->force_host, d->force_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost, d->stream));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(256);
+  cfg.stream = d->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  PW_TRY(cudaLaunchKernelEx(&cfg, force_reduce_kernel, (const double *)d->partials[0], (const double *)d->partials[1],
+                            d->nblocks, d->force_host));
   PW_TRY(cudaEventRecord(d->force_event, d->stream));
   d->force_state = FORCE_ENCODED;
   d->force_step = d->steps;

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(NTHREADS, BLOCKS) aa_step_all(const __grid_con
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (blockIdx.z < s.slices) {
+    if (p.clear_status && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0u) *p.status = 0u;
     uint32_t b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     if (b < s.edge) {
       edge_role<ST, OP, LES, ODD>(p, list, count, b);
@@ -111,6 +112,7 @@ void launch4(const StepParams &p, bool odd, const uint32_t *list, uint32_t count
   if (odd) w.seam = (pairs ? runs : (p.nx + BX - 1u) / BX) * ((seam_rows(p.ny, p.nz) + BY - 1u) / BY);
   const uint32_t slice = gx * gy;
   w.slices = (w.edge + w.floor + w.seam + slice - 1u) / slice;
+  if (p.clear_status && w.slices == 0u) w.slices = 1u;  // its first thread clears the flag
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(gx, gy, p.nz - 2u * off + w.slices);
   cfg.blockDim = dim3(BX, BY);
