@@ -176,6 +176,7 @@ struct pw_domain {
   uint32_t stride = 0;
   size_t esize = 4;
   int device = 0;                 // current device at creation: the domain's memory and streams live there
+  void *arena = nullptr;          // the allocation that holds the arrays below but for edges
   void *f = nullptr;
   float4 *macros = nullptr;
   float4 *plane[2] = {nullptr, nullptr};
@@ -378,6 +379,27 @@ void destroy_side(pw_domain *d) {
   d->side = pwfast::SideStream();
 }
 
+void drop_graphs(pw_domain *d) {
+  for (auto &kv : d->graphs) cudaGraphExecDestroy(kv.second);
+  d->graphs.clear();
+}
+
+// Everything a domain holds, complete or not, once its queued work is done.
+void release_domain(pw_domain *d) {
+  if (d->stream) cudaStreamSynchronize(d->stream);
+  drop_graphs(d);
+  cudaFree(d->arena);
+  cudaFree(d->edges);
+  cudaFree(d->scratch);
+  cudaFree(d->wall_dist);
+  if (d->force_host) pinned_release(d->force_host);
+  if (d->force_event) cudaEventDestroy(d->force_event);
+  destroy_side(d);
+  if (d->stream) cudaStreamDestroy(d->stream);
+  cudaGetLastError();
+  delete d;
+}
+
 int ensure_scratch(pw_domain *d) {
   if (d->scratch) return PW_OK;
   PW_TRY(cudaMalloc(&d->scratch, (size_t)19 * d->cells * 4));
@@ -387,11 +409,6 @@ int ensure_scratch(pw_domain *d) {
 bool alive(const pw_domain *d) {
   if (!d) { set_error("The solver handle is NULL."); return false; }
   return true;
-}
-
-void drop_graphs(pw_domain *d) {
-  for (auto &kv : d->graphs) cudaGraphExecDestroy(kv.second);
-  d->graphs.clear();
 }
 
 // A captured run of kGraphChunk steps beginning at an odd (parity 1) or even step.
@@ -429,12 +446,12 @@ size_t edge_blocks(const pw_domain *d) {
   return d->edge_count ? (d->edge_count + pw::kBlockX * pw::kBlockY - 1) / (pw::kBlockX * pw::kBlockY) : 1;
 }
 
-int build_edge_list(pw_domain *d, Allocs &a) {
+int build_edge_list(pw_domain *d) {
   const uint32_t cells = (uint32_t)d->cells;
   const uint32_t nblk = (cells + kEdgeBlock - 1) / kEdgeBlock;
   const int floor = d->floor_rows ? 1 : 0;
   uint32_t *counts = nullptr, total[2] = {0u, 0u};
-  cudaError_t e = cudaMalloc((void **)&counts, (2 * (size_t)nblk + 2) * 4);
+  cudaError_t e = cudaMallocAsync((void **)&counts, (2 * (size_t)nblk + 2) * 4, d->stream);
   if (e != cudaSuccess) return cuda_status(e, "pw_domain_create edge list");
   for (int part = 0; part <= floor; part++) {
     uint32_t *c = counts + (size_t)part * (nblk + 1);
@@ -444,13 +461,15 @@ int build_edge_list(pw_domain *d, Allocs &a) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(&total[part], c + nblk, 4, cudaMemcpyDeviceToHost, d->stream);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
-  if (e == cudaSuccess) e = a.alloc((void **)&d->edges, ((size_t)total[0] + total[1]) * 4);
+  if (e == cudaSuccess) {
+    const size_t bytes = ((size_t)total[0] + total[1]) * 4;
+    e = cudaMalloc((void **)&d->edges, bytes ? bytes : 16);
+  }
   for (int part = 0; part <= floor && e == cudaSuccess; part++)
     edge_write_kernel<<<nblk, kEdgeBlock, 0, d->stream>>>(d->flags, d->special, d->nx, d->ny, d->nz, cells, floor,
                                                           part, counts + (size_t)part * (nblk + 1),
                                                           d->edges + (part ? total[0] : 0u));
-  if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
-  cudaFree(counts);
+  cudaFreeAsync(counts, d->stream);
   if (e != cudaSuccess) return cuda_status(e, "pw_domain_create edge list");
   d->edge_count = total[0] + total[1];
   d->edge_own = total[0];
@@ -573,7 +592,6 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   }
   size_t plane_n = (size_t)d->ny * d->nz;
 
-  Allocs a;
   cudaError_t e = cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d->force_event, cudaEventDisableTiming);
   // the side stream takes the highest priority, so the edge kernel's few blocks
@@ -585,31 +603,35 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d->side.join, cudaEventDisableTiming);
   // The fast step's two-cell kernel reads (and discards) elements up to
   // nx * ny + nx + 64 past the 19 direction planes.
-  if (e == cudaSuccess)
-    e = a.alloc(&d->f, ((size_t)19 * d->stride + (size_t)d->nx * d->ny + d->nx + 64) * d->esize);
-  if (e == cudaSuccess) e = a.alloc((void **)&d->macros, cells * sizeof(float4));
-  if (e == cudaSuccess) e = a.alloc((void **)&d->plane[0], plane_n * sizeof(float4));
-  if (e == cudaSuccess) e = a.alloc((void **)&d->plane[1], plane_n * sizeof(float4));
-  if (e == cudaSuccess) e = a.alloc((void **)&d->flags, cells * 4);
-  if (e == cudaSuccess) e = a.alloc((void **)&d->special, ((cells + 31) / 32 + 1) * 4);
+  Arena a;
+  a.want(&d->f, ((size_t)19 * d->stride + (size_t)d->nx * d->ny + d->nx + 64) * d->esize);
+  a.want((void **)&d->macros, cells * sizeof(float4));
+  a.want((void **)&d->flags, cells * 4);
+  a.want((void **)&d->special, ((cells + 31) / 32 + 1) * 4);
   d->interp = desc->walls == PW_WALLS_BOUZIDI;
-  if (d->interp && e == cudaSuccess) e = a.alloc((void **)&d->qoff, cells * 4);
-  if (d->interp && e == cudaSuccess) e = a.alloc((void **)&d->qfrac, (grid->nfrac ? grid->nfrac : 1) * 4);
-  if (d->interp && e == cudaSuccess) e = a.alloc(&d->hist, (grid->nfrac ? grid->nfrac : 1) * d->esize);
-  if (e == cudaSuccess) e = a.alloc((void **)&d->partials[0], d->nblocks * 3 * sizeof(double));
-  if (e == cudaSuccess) e = a.alloc((void **)&d->partials[1], d->nblocks * 3 * sizeof(double));
-  if (e == cudaSuccess) e = a.alloc((void **)&d->status_dev, 16);
-  if (e == cudaSuccess) e = a.alloc((void **)&d->totals_dev, 4 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&d->force_host, 4 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&d->status_host, 16);
+  if (d->interp) {
+    a.want((void **)&d->qoff, cells * 4);
+    a.want((void **)&d->qfrac, (grid->nfrac ? grid->nfrac : 1) * 4);
+    a.want(&d->hist, (grid->nfrac ? grid->nfrac : 1) * d->esize);
+  }
+  // from here on: cleared at the start
+  const size_t clear_from = a.total;
+  a.want((void **)&d->partials[0], d->nblocks * 3 * sizeof(double));
+  a.want((void **)&d->partials[1], d->nblocks * 3 * sizeof(double));
+  a.want((void **)&d->plane[0], plane_n * sizeof(float4));
+  a.want((void **)&d->plane[1], plane_n * sizeof(float4));
+  a.want((void **)&d->status_dev, 16);
+  a.want((void **)&d->totals_dev, 4 * sizeof(double));
+  if (e == cudaSuccess) e = a.alloc(&d->arena);
+  if (e == cudaSuccess) {
+    char *slot = static_cast<char *>(pinned_acquire());
+    if (!slot) e = cudaErrorMemoryAllocation;
+    d->force_host = reinterpret_cast<double *>(slot);
+    d->status_host = reinterpret_cast<uint32_t *>(slot ? slot + 4 * sizeof(double) : nullptr);
+  }
   if (e != cudaSuccess) {
     int rc = cuda_status(e, "pw_domain_create");
-    if (d->force_host) cudaFreeHost(d->force_host);
-    if (d->status_host) cudaFreeHost(d->status_host);
-    if (d->force_event) cudaEventDestroy(d->force_event);
-    destroy_side(d);
-    if (d->stream) cudaStreamDestroy(d->stream);
-    delete d;
+    release_domain(d);
     return rc;
   }
   cudaStream_t s = d->stream;
@@ -620,11 +642,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
     cudaMemcpyAsync(d->qoff, grid->qoff, cells * 4, cudaMemcpyDeviceToDevice, s);
     if (grid->nfrac) cudaMemcpyAsync(d->qfrac, grid->fractions, grid->nfrac * 4, cudaMemcpyDeviceToDevice, s);
   }
-  cudaMemsetAsync(d->partials[0], 0, d->nblocks * 3 * sizeof(double), s);
-  cudaMemsetAsync(d->partials[1], 0, d->nblocks * 3 * sizeof(double), s);
-  cudaMemsetAsync(d->plane[0], 0, plane_n * sizeof(float4), s);
-  cudaMemsetAsync(d->plane[1], 0, plane_n * sizeof(float4), s);
-  cudaMemsetAsync(d->status_dev, 0, 16, s);
+  cudaMemsetAsync(static_cast<char *>(d->arena) + clear_from, 0, a.total - clear_from, s);
   if (d->slip)
     clear_slip_links_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(d->flags, d->nx, d->ny, d->nz, d->slip,
                                                                            cells);
@@ -652,7 +670,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   if (!d->tiled && !desc->strict) {
     d->split = true;
     d->one_launch = pwall::step_all_supported(d->nx, d->ny, d->nz, desc->storage, desc->les, d->slip);
-    rc = build_edge_list(d, a);
+    rc = build_edge_list(d);
   }
   if (rc == PW_OK) rc = launch_init(d);
   if (rc == PW_OK) {
@@ -660,15 +678,9 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
     if (e != cudaSuccess) rc = cuda_status(e, "pw_domain_create init");
   }
   if (rc != PW_OK) {
-    cudaFreeHost(d->force_host);
-    cudaFreeHost(d->status_host);
-    cudaEventDestroy(d->force_event);
-    destroy_side(d);
-    cudaStreamDestroy(d->stream);
-    delete d;
+    release_domain(d);
     return rc;
   }
-  a.keep = true;
   noalloc_prepare_device();
   *out = d;
   return PW_OK;
@@ -676,20 +688,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
 
 void pw_domain_destroy(pw_domain *d) {
   if (!d) return;
-  cudaStreamSynchronize(d->stream);
-  drop_graphs(d);
-  cudaFree(d->f); cudaFree(d->macros); cudaFree(d->plane[0]); cudaFree(d->plane[1]);
-  cudaFree(d->flags); cudaFree(d->special); cudaFree(d->partials[0]); cudaFree(d->partials[1]);
-  cudaFree(d->status_dev); cudaFree(d->totals_dev); cudaFree(d->scratch);
-  cudaFree(d->edges);
-  cudaFree(d->wall_dist);
-  cudaFree(d->qoff); cudaFree(d->qfrac); cudaFree(d->hist);
-  cudaFreeHost(d->force_host); cudaFreeHost(d->status_host);
-  cudaEventDestroy(d->force_event);
-  destroy_side(d);
-  cudaStreamDestroy(d->stream);
-  cudaGetLastError();
-  delete d;
+  release_domain(d);
 }
 
 int pw_reset(pw_domain *d) {

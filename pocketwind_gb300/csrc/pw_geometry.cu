@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "pw_internal.h"
@@ -71,10 +72,59 @@ static void tmp_free(void *p, cudaStream_t s) {
 }
 
 Grid::~Grid() {
-  cudaFree(flags);
-  cudaFree(qoff);
-  cudaFree(fractions);
-  cudaFree(boundary);
+  cudaFree(cell_arrays);
+  cudaFree(link_arrays);
+}
+
+// ------------------------------------------------------------------ pinned slots
+namespace {
+struct PinnedSlab {
+  char *base;
+  uint64_t used;  // a bit a slot
+};
+constexpr size_t kSlabSlots = 64;
+std::mutex g_pinned_lock;
+std::vector<PinnedSlab> g_pinned;
+}  // namespace
+
+void *pinned_acquire() {
+  std::lock_guard<std::mutex> hold(g_pinned_lock);
+  PinnedSlab *slab = nullptr;
+  for (PinnedSlab &s : g_pinned)
+    if (~s.used) { slab = &s; break; }
+  if (!slab) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, kSlabSlots * kPinnedSlot, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_pinned.push_back(PinnedSlab{static_cast<char *>(p), 0});
+    slab = &g_pinned.back();
+  }
+  const int k = __builtin_ctzll(~slab->used);
+  slab->used |= 1ull << k;
+  void *slot = slab->base + (size_t)k * kPinnedSlot;
+  std::memset(slot, 0, kPinnedSlot);
+  return slot;
+}
+
+void pinned_release(void *slot) {
+  std::lock_guard<std::mutex> hold(g_pinned_lock);
+  bool other_empty = false;
+  size_t at = g_pinned.size();
+  for (size_t i = 0; i < g_pinned.size(); i++) {
+    const ptrdiff_t off = static_cast<char *>(slot) - g_pinned[i].base;
+    if (off >= 0 && off < (ptrdiff_t)(kSlabSlots * kPinnedSlot)) {
+      g_pinned[i].used &= ~(1ull << (off / (ptrdiff_t)kPinnedSlot));
+      at = i;
+    } else if (!g_pinned[i].used) {
+      other_empty = true;
+    }
+  }
+  if (at < g_pinned.size() && !g_pinned[at].used && other_empty) {
+    cudaFreeHost(g_pinned[at].base);
+    g_pinned.erase(g_pinned.begin() + (ptrdiff_t)at);
+  }
 }
 
 // ------------------------------------------------------------------ scan
@@ -833,7 +883,6 @@ static int finish_grid(pw_grid *g, const uint8_t *body, const uint8_t *sup, int 
   GridInfo got{};
   cudaError_t e = tmp_alloc(&sums, 2 * (size_t)blocks * 4, s);
   if (e == cudaSuccess) e = tmp_alloc(&marked, 2 * rows, s);
-  if (e == cudaSuccess) e = cudaMalloc(&g->qoff, cells * 4);
   int rc = e == cudaSuccess ? PW_OK : cuda_status(e, "voxelize counts");
   if (rc == PW_OK) {
     cudaMemsetAsync(marked, 0, 2 * rows, s);
@@ -845,8 +894,10 @@ static int finish_grid(pw_grid *g, const uint8_t *body, const uint8_t *sup, int 
     rc = read_info(info, &got, s);
   }
   if (rc == PW_OK) {
-    e = cudaMalloc(&g->fractions, ((size_t)got.links ? got.links : 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&g->boundary, ((size_t)got.boundary ? got.boundary : 1) * 4);
+    Arena a;
+    a.want((void **)&g->fractions, (size_t)got.links * 4);
+    a.want((void **)&g->boundary, (size_t)got.boundary * 4);
+    e = a.alloc(&g->link_arrays);
     if (e == cudaSuccess && links_out && got.links) e = tmp_alloc(links_out, (size_t)got.links * sizeof(uint2), s);
     if (e != cudaSuccess) rc = cuda_status(e, "voxelize links");
   }
@@ -951,7 +1002,10 @@ int pw_voxelize_opts(const float *body, uint32_t body_triangles, const float *su
   int rc = PW_OK;
   uint8_t *votes[2] = {nullptr, nullptr};
   GridInfo *info = nullptr;
-  cudaError_t e = cudaMalloc(&g->flags, cells * 4);
+  Arena a;
+  a.want((void **)&g->flags, cells * 4);
+  a.want((void **)&g->qoff, cells * 4);
+  cudaError_t e = a.alloc(&g->cell_arrays);
   float *d_sup = nullptr;
   if (e == cudaSuccess) e = tmp_alloc(&info, sizeof(GridInfo), s);
   if (e == cudaSuccess) e = tmp_alloc(&d_mesh, (body_triangles ? body_triangles : 1) * 36, s);
@@ -1023,10 +1077,13 @@ int pw_grid_from_host(uint32_t nx, uint32_t ny, uint32_t nz, const uint32_t *geo
   g->nx = nx; g->ny = ny; g->nz = nz; g->cells = cells;
   unsigned long long *bad = nullptr;
   unsigned long long bad_h = ~0ull;
-  cudaError_t e = cudaMalloc(&g->flags, cells * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&g->qoff, cells * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&g->fractions, (fractions ? fractions : 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&g->boundary, (nboundary ? nboundary : 1) * 4);
+  Arena cell_arrays, link_arrays;
+  cell_arrays.want((void **)&g->flags, cells * 4);
+  cell_arrays.want((void **)&g->qoff, cells * 4);
+  link_arrays.want((void **)&g->fractions, fractions * 4);
+  link_arrays.want((void **)&g->boundary, nboundary * 4);
+  cudaError_t e = cell_arrays.alloc(&g->cell_arrays);
+  if (e == cudaSuccess) e = link_arrays.alloc(&g->link_arrays);
   if (e == cudaSuccess) e = cudaMalloc(&bad, 8);
   if (e == cudaSuccess) e = cudaMemcpyAsync(g->flags, geometry, cells * 4, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(g->qoff, geometry + cells, cells * 4, cudaMemcpyHostToDevice, s);
