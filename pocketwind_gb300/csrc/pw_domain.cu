@@ -27,21 +27,27 @@ namespace {
 
 constexpr int kGraphChunk = 64;  // steps per captured graph
 
-// The special bits, and the first fluid cell into *first_fluid: a warp offers its
-// first one only while it is below the minimum so far, so all but the first few
-// read and go on (an atomic per fluid cell took 2.59 ms at 256x128x128).
+// The special bits, and the first fluid cell into *first_fluid: a block offers its
+// first one only while it is below the minimum so far, so all but the first wave of
+// blocks read and go on (an atomic per fluid cell took 2.59 ms at 256x128x128, one per
+// warp of the first wave 48 us).
 __global__ void special_kernel(const uint32_t *flags, size_t cells, uint32_t *special,
                                unsigned long long *first_fluid) {
+  __shared__ uint32_t first[32];
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t f = i < cells ? flags[i] : (uint32_t)pw::SOLID;
   const uint32_t word = __ballot_sync(0xffffffffu, i < cells && ((f & 7u) != pw::FLUID || (f >> 3) != 0u));
   const uint32_t fluid = __ballot_sync(0xffffffffu, (f & 7u) == pw::FLUID);
-  if ((threadIdx.x & 31) == 0 && i < cells) {
-    special[i >> 5] = word;
-    if (fluid) {
-      const unsigned long long n = i + (unsigned long long)(__ffs(fluid) - 1);
-      if (n < *(volatile unsigned long long *)first_fluid) atomicMin(first_fluid, n);
-    }
+  if ((threadIdx.x & 31) == 0) {
+    if (i < cells) special[i >> 5] = word;
+    first[threadIdx.x >> 5] = fluid ? threadIdx.x + (uint32_t)__ffs(fluid) - 1u : ~0u;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t k = ~0u;
+    for (uint32_t w = 0; w < blockDim.x / 32; w++) k = min(k, first[w]);
+    const unsigned long long n = (unsigned long long)blockIdx.x * blockDim.x + k;
+    if (k != ~0u && n < *(volatile unsigned long long *)first_fluid) atomicMin(first_fluid, n);
   }
 }
 

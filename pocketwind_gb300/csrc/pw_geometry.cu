@@ -343,13 +343,21 @@ __global__ void __launch_bounds__(kRasterThreads) raster_kernel(const float *mes
   }
 }
 
-// Sorts each column's hits and adds its spans [ceil(h0), ceil(h1)) to the votes,
-// one projection a launch (the projections' columns share cells).  Threads run
-// over the columns with x the fastest of (u, v); columns along x are filled by
-// the whole warp, one lane's span at a time, so that each store is a line.
-__global__ void __launch_bounds__(128) column_kernel(Proj P, const uint32_t *offset, double *hits, uint8_t *votes,
-                                                     uint32_t *odd) {
+// Sorts each column's hits and adds its spans [ceil(h0), ceil(h1)) to the votes, the
+// projections side by side (blockIdx.y): a vote is one added to its byte of a word, and
+// nothing waits for the sum: 8 us at 256x128x128 (a load, an increment and a store a
+// cell, one projection after another, took 82 us, each lane waiting for its last cell).
+// Threads run over the columns with x the fastest of (u, v); columns along x are filled
+// by the whole warp, one lane's span at a time, a word of four cells a lane.
+__device__ __forceinline__ void add_vote(uint32_t *votes, size_t cell) {
+  atomicAdd(&votes[cell >> 2], 1u << (8u * (uint32_t)(cell & 3u)));
+}
+
+__global__ void __launch_bounds__(128) column_kernel(Projs projs, const uint32_t *offset, double *hits,
+                                                     uint32_t *votes, uint32_t *odd) {
+  const Proj &P = projs.p[blockIdx.y];
   const size_t ncol = (size_t)P.su * P.sv, id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((size_t)blockIdx.x * blockDim.x >= ncol) return;
   const uint32_t lane = threadIdx.x & 31u;
   const bool along_x = P.axis == 0, v_is_x = P.v == 0;
   uint32_t u = 0, v = 0, n = 0, at = 0;
@@ -376,14 +384,20 @@ __global__ void __launch_bounds__(128) column_kernel(Proj P, const uint32_t *off
       s1 = (long long)fmin((double)P.sa, ceil(h[pair + 1]));
     }
     if (!along_x) {
-      for (long long c = s0; c < s1; c++) votes[base + (size_t)c * P.sta]++;
+      for (long long c = s0; c < s1; c++) add_vote(votes, base + (size_t)c * P.sta);
       continue;
     }
     for (uint32_t left = __ballot_sync(0xffffffffu, s0 < s1); left; left &= left - 1u) {
       const int src = __ffs(left) - 1;
       const long long a = __shfl_sync(0xffffffffu, s0, src), b = __shfl_sync(0xffffffffu, s1, src);
       const size_t row = __shfl_sync(0xffffffffu, (unsigned long long)base, src);
-      for (long long c = a + lane; c < b; c += 32) votes[row + (size_t)c]++;
+      const size_t from = row + (size_t)a, to = row + (size_t)b;  // cells, a word of four a lane
+      for (size_t w = (from >> 2) + lane; w <= (to - 1) >> 2; w += 32) {
+        uint32_t add = 0x01010101u;
+        if (4 * w < from) add &= 0xffffffffu << (8u * (uint32_t)(from - 4 * w));
+        if (4 * w + 4 > to) add &= 0xffffffffu >> (8u * (uint32_t)(4 * w + 4 - to));
+        atomicAdd(&votes[w], add);
+      }
     }
   }
 }
@@ -433,13 +447,16 @@ __global__ void sum_rows_kernel(const uint8_t *v, size_t rows, uint32_t *out) {
 // arithmetic and no per-cell counts this pass, the packing pass and their scan
 // take the place of six passes (134 us for the masks alone, with 64-bit
 // remainders, and 103 us for the counts' scans, the q offsets, the fractions
-// and the boundary list, at 256x128x128).
+// and the boundary list, at 256x128x128).  Where none of the nine rows around a cell
+// holds a wall (wall_rows, the same bytes for a whole warp) its 18 neighbours are not
+// read.
 constexpr uint32_t kBodyBit = 1u << 31;
 constexpr uint32_t kLinkBits = 0x3ffff0u;
 constexpr int kMaskThreads = 256, kMaskCells = 4 * kMaskThreads;
 
 __global__ void __launch_bounds__(kMaskThreads) wall_mask_kernel(uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz,
-                                                                int floor_on, uint32_t *sums, uint32_t blocks) {
+                                                                int floor_on, const uint8_t *wall_rows, uint32_t *sums,
+                                                                uint32_t blocks) {
   __shared__ uint32_t total[2];
   if (threadIdx.x < 2) total[threadIdx.x] = 0u;
   __syncthreads();
@@ -452,6 +469,11 @@ __global__ void __launch_bounds__(kMaskThreads) wall_mask_kernel(uint32_t *flags
     const uint32_t i = (uint32_t)at, f = flags[at];
     if ((f & 7u) != pw::FLUID) continue;
     const uint32_t row = i / nx, x = i - row * nx, z = row / ny, y = row - z * ny;
+    const uint32_t rm = y == 0 ? ny - 1 : y - 1, rp = y + 1 == ny ? 0 : y + 1;
+    const uint32_t pm = (z == 0 ? nz - 1 : z - 1) * ny, p0 = z * ny, pp = (z + 1 == nz ? 0 : z + 1) * ny;
+    uint32_t walls = wall_rows[pm + rm] | wall_rows[pm + y] | wall_rows[pm + rp] | wall_rows[p0 + rm] | wall_rows[row] |
+                     wall_rows[p0 + rp] | wall_rows[pp + rm] | wall_rows[pp + y] | wall_rows[pp + rp];
+    if (!walls && !(floor_on && z <= 1u)) continue;
     // offsets to the source of each axis' step (mod 2^32, as the cell index)
     const uint32_t ym = y == 0 ? plane - nx : 0u - nx, yp = y + 1 == ny ? nx - plane : nx;
     const uint32_t span = plane * nz;
@@ -560,7 +582,7 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
   uint32_t *count = nullptr, *offset = nullptr;
   GridInfo got{};
   double *hits = nullptr;
-  cudaError_t e = tmp_alloc(votes_out, cells, s);
+  cudaError_t e = tmp_alloc(votes_out, (cells + 3) / 4 * 4, s);
   uint8_t *votes = *votes_out;
   if (e == cudaSuccess) e = tmp_alloc(&count, ncol * 4, s);
   if (e == cudaSuccess) e = tmp_alloc(&offset, (ncol + 1) * 4, s);
@@ -570,7 +592,7 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
   const uint32_t slices = std::max(1u, std::min(1024u, 152u * 16u / groups));
   const unsigned rblocks = (unsigned)(((uint64_t)groups * slices + kRasterThreads / 32 - 1) / (kRasterThreads / 32));
   if (rc == PW_OK) {
-    cudaMemsetAsync(votes, 0, cells, s);
+    cudaMemsetAsync(votes, 0, (cells + 3) / 4 * 4, s);
     cudaMemsetAsync(count, 0, ncol * 4, s);
     raster_kernel<false><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, nullptr, nullptr,
                                                             &info->nonfinite);
@@ -586,9 +608,10 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
     if (e != cudaSuccess) rc = cuda_status(e, "voxelize hits");
     if (rc == PW_OK) {
       raster_kernel<true><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, offset, hits, nullptr);
-      for (int p = 0; p < 3; p++)
-        column_kernel<<<nblk((size_t)P.p[p].su * P.p[p].sv, 128), 128, 0, s>>>(P.p[p], offset, hits, votes,
-                                                                               &info->odd[which]);
+      size_t most = 0;
+      for (int p = 0; p < 3; p++) most = std::max(most, (size_t)P.p[p].su * P.p[p].sv);
+      column_kernel<<<dim3(nblk(most, 128), 3), 128, 0, s>>>(P, offset, hits, reinterpret_cast<uint32_t *>(votes),
+                                                             &info->odd[which]);
     }
   }
   tmp_free(count, s); tmp_free(offset, s); tmp_free(hits, s);
@@ -691,7 +714,7 @@ __device__ __forceinline__ double from_ordered(unsigned long long k) {
 // linkFraction of every wall link: FLOOR links keep 1/2; SOLID links cast against
 // the body, SUPPORT links against the supports; a miss keeps 1/2 and counts; hits
 // clamp to [1e-3, 1].
-// A warp takes 32 consecutive links, which share most of their bins.  For one
+// A warp takes eight consecutive links, which share most of their bins.  For one
 // link after another all lanes scan its bins' triangles (nearestLinkHit,
 // triangle-bins.ts:136-161; bins next to each other in x are one range) with the
 // box test in binary32: the segment's ends are whole numbers, rounded toward the
@@ -699,8 +722,11 @@ __device__ __forceinline__ double from_ordered(unsigned long long k) {
 // to a queue, and the binary64 intersections run for 32 queued pairs at a time:
 // binary64 issues at the same rate for one lane as for 32.  A thread per cell
 // with its links and triangles in turn took 4.92 ms for the 70,000 links of a
-// 150x75x61 grid with 12,288 triangles; this form takes 0.21 ms.
+// 150x75x61 grid with 12,288 triangles (14,000 of them cast, the others on the floor).
+// With 32 links a warp there were too few warps to cover the loads (210 us); eight take
+// 92 us.
 constexpr int kLinkThreads = 128;
+constexpr uint32_t kWarpLinks = 8;
 struct LinkCast { int ox, oy, oz, dir; };
 __global__ void __launch_bounds__(kLinkThreads) link_fraction_kernel(const uint32_t *flags, const uint2 *links,
                                                                     uint32_t nlinks, float *fractions, uint32_t nx,
@@ -710,9 +736,9 @@ __global__ void __launch_bounds__(kLinkThreads) link_fraction_kernel(const uint3
   __shared__ unsigned long long best[kLinkThreads / 32][32];
   __shared__ uint2 queue[kLinkThreads / 32][64];  // (triangle, link's lane), bit 5 of the lane: the supports
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint32_t first = (blockIdx.x * (kLinkThreads / 32) + w) * 32u;
+  const uint32_t first = (blockIdx.x * (kLinkThreads / 32) + w) * kWarpLinks;
   if (first >= nlinks) return;  // the whole warp
-  const uint32_t link = first + lane;
+  const uint32_t link = lane < kWarpLinks ? first + lane : nlinks;
   uint32_t target = 0;  // 1 the body, 2 the supports: this lane's link is cast
   LinkCast c = {0, 0, 0, 0};
   bool hit = link < nlinks;  // until a cast misses
@@ -855,7 +881,7 @@ static int measure_links(pw_grid *g, const float *d_body, uint32_t nbody, const 
   if (rc == PW_OK && has_sup) rc = build_bins(d_sup, nsup, g->nx, g->ny, g->nz, &sup, s);
   if (rc == PW_OK) {
     const uint32_t n = (uint32_t)g->nfrac;
-    link_fraction_kernel<<<nblk(n, kLinkThreads), kLinkThreads, 0, s>>>(g->flags, links, n, g->fractions, g->nx, g->ny,
+    link_fraction_kernel<<<nblk(n, kWarpLinks * (kLinkThreads / 32)), kLinkThreads, 0, s>>>(g->flags, links, n, g->fractions, g->nx, g->ny,
                                                                         g->nz, body, sup, has_sup ? 1 : 0, &info->missed);
     rc = read_info(info, &got, s);
   }
@@ -889,7 +915,7 @@ static int finish_grid(pw_grid *g, const uint8_t *body, const uint8_t *sup, int 
     kinds_kernel<<<nblk(cells), 256, 0, s>>>(body, sup, g->flags, g->nx, g->ny, g->nz, floor_on, &info->solid, marked,
                                              marked + rows);
     sum_rows_kernel<<<nblk(rows), 256, 0, s>>>(marked, rows, &info->frontal);
-    wall_mask_kernel<<<blocks, kMaskThreads, 0, s>>>(g->flags, g->nx, g->ny, g->nz, floor_on, sums, blocks);
+    wall_mask_kernel<<<blocks, kMaskThreads, 0, s>>>(g->flags, g->nx, g->ny, g->nz, floor_on, marked + rows, sums, blocks);
     scan_offsets<<<2, kScanThreads, 0, s>>>(sums, blocks, &info->links, nullptr);
     rc = read_info(info, &got, s);
   }
