@@ -261,16 +261,18 @@ PW_API int pw_checkpoint_load(pw_domain *dom, const void *in, size_t size);
    the reference runs one solver at a time, src/app/solver-slot.ts) ----
    Members are domains of the fast build's one-cell-per-thread path sharing
    storage, operator and LES, with equal step counts and no ramp in progress.
-   Each batch step is two persistent launches, one over all members' plain
-   cells and one over their seam and edge cells running beside it, replayed
-   from captured CUDA graphs; members keep their own force, macro and readout
+   Members step by their own launches side by side on their streams, or, with
+   few cells each or a step that is not one launch, by two persistent launches
+   a step, one over all members' plain cells and one over their seam and edge
+   cells running beside it, replayed from captured CUDA graphs; members keep their own force, macro and readout
    calls, which wait for the batch's queued steps.  A member must not be
    stepped on its own while it belongs to a batch. */
 typedef struct pw_batch pw_batch;
 typedef struct {
   uint32_t blocks;         /* persistent grid chosen */
   uint32_t rows_per_item;  /* plain rows per work item chosen */
-  float ms_per_step;       /* its measured time per step */
+  float ms_per_step;       /* measured time per step of what is kept: that shape, or
+                              the members' own launches where those are faster */
   uint32_t candidates;     /* launch shapes timed */
 } pw_batch_tuning;
 PW_API int pw_batch_create(pw_domain *const *members, uint32_t count, pw_batch **out);

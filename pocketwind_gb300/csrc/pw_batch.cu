@@ -1,7 +1,9 @@
-// Batched stepping of many independent domains: two concurrent persistent
-// launches per step over the work of every member, replayed from captured CUDA
-// graphs, with the launch shape chosen by timing (pw_batch_tune).  No counterpart in the
-// reference, which runs one solver at a time (src/app/solver-slot.ts).
+// Batched stepping of many independent domains.  No counterpart in the reference, which
+// runs one solver at a time (src/app/solver-slot.ts).  Members whose step is one launch
+// take their own steps side by side on their streams (queue_own).  The others, members of
+// few cells, and where tuning finds it faster: two concurrent persistent launches per step
+// over the work of every member, replayed from captured CUDA graphs, with the launch shape
+// chosen by timing (pw_batch_tune).
 //
 // Work items (per step parity):
 //   plain  R rows x 64 cells of one member (two cells per thread: the 32-bit
@@ -177,7 +179,9 @@ struct pw_batch {
   bool pairs = false;             // every member's nx is even: the plain items use the cell-pair kernel
   const uint32_t **lists = nullptr;
   uint32_t *counts = nullptr;
-  uint32_t rows = 4;       // plain rows per work item
+  bool can_own = false;    // every member's step is one launch
+  bool own = false;        // the members step by their own launches, side by side
+  uint32_t rows = 16;      // plain rows per work item
   unsigned blocks = 0;     // persistent grid
   uint64_t steps = 0;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
@@ -332,7 +336,25 @@ void batch_to_members(pw_batch *b) {
   for (pw_domain *d : b->members) cudaStreamWaitEvent(member_view(d).stream, b->done, 0);
 }
 
+// The members' own steps, each on its stream, in turn: the members do not wait for one
+// another, and a step runs at a single domain's rate (its offsets are kernel constants,
+// no block barriers between items).  A step of 32 mixed tunnels (FP16; FP32): 433 and 622
+// us, as the tuned persistent launches 493 and 736; of eight 101x53x47: 40 and 62 against
+// 68 and 78; of 64 tunnels of 64x32x32: 98 and 148 against 99 and 152.  Four or 16 steps
+// of a member at a time: the mixed tunnels 2% slower, 24 of 96x48x48 3 to 7% faster.
+void queue_own(pw_batch *b, uint64_t count, int macro_last) {
+  for (uint64_t k = 0; k < count; k++)
+    for (pw_domain *d : b->members)
+      member_enqueue(d, b->steps + 1 + k, macro_last && k + 1 == count, macro_last && k + 2 == count, k > 0);
+  b->steps += count;
+}
+
 int queue_steps(pw_batch *b, uint64_t count, int macro_last) {
+  if (b->own) {
+    queue_own(b, count, macro_last);
+    PW_TRY(cudaGetLastError());
+    return PW_OK;
+  }
   uint64_t k = 0;
   while (count - k >= (uint64_t)kChunk) {
     const int macro = macro_last && count - k == (uint64_t)kChunk;
@@ -395,8 +417,17 @@ int pw_batch_create(pw_domain *const *members, uint32_t count, pw_batch **out) {
   for (uint32_t m = 0; m < count; m++) b->pairs = b->pairs && (member_view(members[m]).nx & 1u) == 0u;
   b->storage = first.storage; b->op = first.op; b->les = first.les;
   b->steps = first.steps;
+  b->can_own = true;
+  uint64_t cells = 0;
+  for (uint32_t m = 0; m < count; m++) {
+    const MemberView v = member_view(members[m]);
+    b->can_own = b->can_own && v.one_launch;
+    cells += (uint64_t)v.nx * v.ny * v.nz;
+  }
+  // below 48 K cells a member a launch outweighs its step (64x32x32, 65 K cells: even)
+  b->own = b->can_own && cells >= (uint64_t)count * (48u << 10);
   b->sms = (unsigned)max_blocks();
-  b->blocks = b->sms * 4u;
+  b->blocks = b->sms * 32u;  // with 16 rows an item what tuning mostly finds (4 and 4: half the rate)
   auto fail = [&](int rc) {
     pw_batch_destroy(b);
     return rc;
@@ -466,9 +497,9 @@ int pw_batch_step(pw_batch *b, uint64_t count, int write_macro_on_last) {
       return PW_ERR_INVALID;
     }
   if (count == 0) return PW_OK;
-  members_to_batch(b);
+  if (!b->own) members_to_batch(b);
   int rc = queue_steps(b, count, write_macro_on_last);
-  batch_to_members(b);
+  if (!b->own) batch_to_members(b);
   for (pw_domain *d : b->members) member_advance(d, count);
   return rc;
 }
@@ -480,10 +511,12 @@ int pw_batch_time_steps(pw_batch *b, uint64_t count, float *ms) {
   PW_TRY(cudaEventCreate(&t1));
   members_to_batch(b);
   cudaEventRecord(t0, b->stream);
+  if (b->own) batch_to_members(b);  // the members start after t0
   int rc = PW_OK;
   for (pw_domain *d : b->members)
     if (member_view(d).steps != b->steps) rc = PW_ERR_INVALID;
   if (rc == PW_OK) rc = queue_steps(b, count, 0);
+  if (b->own) members_to_batch(b);  // t1 after every member's last step
   cudaEventRecord(t1, b->stream);
   batch_to_members(b);
   if (rc == PW_OK)
@@ -499,7 +532,8 @@ int pw_batch_time_steps(pw_batch *b, uint64_t count, float *ms) {
 
 // Time every candidate launch shape (persistent grid of 2, 4, 8, 16 or 32 blocks
 // per SM, and 8, 16, 32 or 64 plain rows per work item) over `trial_steps` real
-// steps each (an even number, after two warm-up steps) and keep the fastest.
+// steps each (an even number, after two warm-up steps) and keep the fastest, then
+// the members' own launches, which are taken where they are faster than it.
 // The trial steps advance the members.
 int pw_batch_tune(pw_batch *b, uint32_t trial_steps, pw_batch_tuning *out) {
   if (!b || trial_steps == 0) { set_error("The batch handle is NULL or the trial has no steps."); return PW_ERR_INVALID; }
@@ -507,6 +541,7 @@ int pw_batch_tune(pw_batch *b, uint32_t trial_steps, pw_batch_tuning *out) {
   const unsigned sms = (unsigned)max_blocks();
   const unsigned grid_mult[] = {2, 4, 8, 16, 32};
   const uint32_t row_opts[] = {8, 16, 32, 64};
+  b->own = false;
   float best = 1e30f;
   unsigned best_blocks = b->blocks;
   uint32_t best_rows = b->rows, tried = 0;
@@ -532,6 +567,15 @@ int pw_batch_tune(pw_batch *b, uint32_t trial_steps, pw_batch_tuning *out) {
   drop_graphs(b);
   int rc = build_segments(b);
   if (rc != PW_OK) return rc;
+  if (b->can_own) {
+    b->own = true;
+    rc = pw_batch_step(b, 2, 0);
+    float ms = 0.0f;
+    if (rc == PW_OK) rc = pw_batch_time_steps(b, trial_steps, &ms);
+    if (rc != PW_OK) return rc;
+    b->own = ms < best;
+    best = std::min(best, ms);
+  }
   if (out) {
     out->blocks = best_blocks;
     out->rows_per_item = best_rows;

@@ -289,7 +289,7 @@ pw::StepParams params_for(const pw_domain *d, uint64_t step, float u_in, int wri
 // macro step starts at zero: a step of one launch before it in the same call clears it
 // (before_macro, then cleared), without a memset between the two.
 void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool before_macro = false,
-                  bool cleared = false) {
+                  bool cleared = false, bool early = true) {
   pw::StepParams p = params_for(d, step, u_in, write_macro);
   const bool one = d->one_launch && d->split && !d->closure_frag;
   p.clear_status = one && before_macro ? 1 : 0;
@@ -310,7 +310,8 @@ void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool
     pwclosure_host::launch_closure_step(p, d->desc.storage, d->desc.op, odd, d->grid, d->closure_frag, d->wall_dist,
                                         d->stream);
   else if (d->one_launch && d->split)
-    pwall::launch_step_all(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->edges, d->edge_own, d->stream);
+    pwall::launch_step_all(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->edges, d->edge_own, d->stream,
+                           early);
   else if (d->split)
     pwfast::launch_step_split(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->plain_grid, d->edges,
                               d->edge_own, d->stream, nullptr, &d->side);
@@ -957,6 +958,7 @@ namespace pwhost {
 MemberView member_view(const pw_domain *d) {
   MemberView v;
   v.split = d->split;
+  v.one_launch = d->one_launch;
   v.closure = d->closure_frag != nullptr;
   v.storage = d->desc.storage;
   v.op = d->desc.op;
@@ -976,6 +978,9 @@ pw::StepParams member_params(const pw_domain *d, uint64_t step, int write_macro)
   pw::StepParams p = params_for(d, step, d->u_in, write_macro);
   p.floor_rows = 0;  // a batch's edge items take the floor layer through the general path
   return p;
+}
+void member_enqueue(pw_domain *d, uint64_t step, int write_macro, bool before_macro, bool cleared) {
+  enqueue_step(d, step, d->u_in, write_macro, before_macro, cleared, false);
 }
 void member_advance(pw_domain *d, uint64_t n) { d->steps += n; }
 }  // namespace pwhost

@@ -44,6 +44,7 @@ void noalloc_prepare_device();
 // What a batch needs of a member domain (pw_batch.cu).
 struct MemberView {
   bool split;                // fast build, one cell per thread (plain kernels + edge list)
+  bool one_launch;           // its step is one launch
   bool closure;              // a learned closure is attached
   int storage, op, les;
   uint32_t nx, ny, nz;
@@ -59,6 +60,9 @@ struct MemberView {
 MemberView member_view(const pw_domain *d);
 // The step parameters of step `step` (1-based) at the domain's full inlet speed.
 pw::StepParams member_params(const pw_domain *d, uint64_t step, int write_macro);
+// Queue step `step` of a one-launch domain on its own stream, among other domains'
+// steps; write_macro and before_macro as in pw_domain.cu's enqueue_step.
+void member_enqueue(pw_domain *d, uint64_t step, int write_macro, bool before_macro, bool cleared);
 // Count `n` steps run for the domain by a batch.
 void member_advance(pw_domain *d, uint64_t n);
 

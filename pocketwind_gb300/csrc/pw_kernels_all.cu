@@ -100,7 +100,7 @@ namespace {
 constexpr int kPairBlocks = 8, kCellBlocks = 7, kLinearBlocks = 7;
 
 template <int ST, int OP, bool LES, Plain FORM>
-void launch4(const StepParams &p, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s) {
+void launch4(const StepParams &p, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s, bool early) {
   const bool linear = FORM == LINEAR || FORM == LINEAR_NY_ODD, pairs = FORM == PAIRS;
   const uint32_t off = odd ? 1u : 0u, runs = (p.nx + 2u * BX - 1u) / (2u * BX);
   // pairs of a plane, one more when it starts at an odd cell
@@ -121,28 +121,29 @@ void launch4(const StepParams &p, bool odd, const uint32_t *list, uint32_t count
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   constexpr int B = FORM == RUNS ? kCellBlocks : (FORM == PAIRS ? kPairBlocks : kLinearBlocks);
   if (odd) cudaLaunchKernelEx(&cfg, aa_step_all<ST, OP, LES, true, FORM, B>, p, list, count, w);
   else cudaLaunchKernelEx(&cfg, aa_step_all<ST, OP, LES, false, FORM, B>, p, list, count, w);
 }
 
 template <int ST, bool LES, Plain FORM>
-void launch3(const StepParams &p, int op, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s) {
-  if (op == OP_REG) launch4<ST, OP_REG, LES, FORM>(p, odd, list, count, s);
-  else launch4<ST, OP_TRT, LES, FORM>(p, odd, list, count, s);
+void launch3(const StepParams &p, int op, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s, bool early) {
+  if (op == OP_REG) launch4<ST, OP_REG, LES, FORM>(p, odd, list, count, s, early);
+  else launch4<ST, OP_TRT, LES, FORM>(p, odd, list, count, s, early);
 }
 
 // 16-bit storage: pairs of a row, or of a plane with nx odd (without LES).
 template <int ST>
-void launch2(const StepParams &p, int op, int les, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s) {
+void launch2(const StepParams &p, int op, int les, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s,
+             bool early) {
   if ((p.nx & 1u) == 0u) {
-    if (les) launch3<ST, true, PAIRS>(p, op, odd, list, count, s);
-    else launch3<ST, false, PAIRS>(p, op, odd, list, count, s);
+    if (les) launch3<ST, true, PAIRS>(p, op, odd, list, count, s, early);
+    else launch3<ST, false, PAIRS>(p, op, odd, list, count, s, early);
   } else if (p.ny & 1u) {
-    launch3<ST, false, LINEAR_NY_ODD>(p, op, odd, list, count, s);
+    launch3<ST, false, LINEAR_NY_ODD>(p, op, odd, list, count, s, early);
   } else {
-    launch3<ST, false, LINEAR>(p, op, odd, list, count, s);
+    launch3<ST, false, LINEAR>(p, op, odd, list, count, s, early);
   }
 }
 
@@ -163,11 +164,11 @@ bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int 
 }
 
 void launch_step_all(const StepParams &p, int storage, int op, int les, bool odd, const uint32_t *list, uint32_t count,
-                     cudaStream_t s) {
-  if (storage == STORE_F16) launch2<STORE_F16>(p, op, les, odd, list, count, s);
-  else if (storage == STORE_BF16) launch2<STORE_BF16>(p, op, les, odd, list, count, s);
-  else if (les) launch3<STORE_F32, true, RUNS>(p, op, odd, list, count, s);
-  else launch3<STORE_F32, false, RUNS>(p, op, odd, list, count, s);
+                     cudaStream_t s, bool early) {
+  if (storage == STORE_F16) launch2<STORE_F16>(p, op, les, odd, list, count, s, early);
+  else if (storage == STORE_BF16) launch2<STORE_BF16>(p, op, les, odd, list, count, s, early);
+  else if (les) launch3<STORE_F32, true, RUNS>(p, op, odd, list, count, s, early);
+  else launch3<STORE_F32, false, RUNS>(p, op, odd, list, count, s, early);
 }
 
 }  // namespace pwall

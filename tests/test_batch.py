@@ -216,3 +216,37 @@ def test_batch_step_is_deterministic():
     for a, b in zip(runs[0], runs[1]):
         assert np.array_equal(a, b)
 
+
+
+# members of few cells share the persistent launches, larger ones step by their own; odd
+# and even nx, fewer rows than an item holds
+@pytest.mark.gpu
+@pytest.mark.parametrize("layouts", [[(24, 16, 12), (33, 9, 14), (18, 20, 31)], [(24, 16, 12), (30, 16, 12)],
+                                     [(72, 36, 33), (65, 35, 36)]])
+@pytest.mark.parametrize("precision", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("counts", [(1, 2, 3), (51,)])
+def test_batch_forms_match_the_reference(layouts, precision, counts):
+    """f32 populations within the reference's 1e-5 of the binary32 restatement on each
+    member's grid; 16-bit ones within twice the restatement's own 16-bit distance from it
+    (the bound of test_batched_members_match_the_reference_fp32_path)."""
+    from oracle import oracle as O
+    from pocketwind_gb300 import geometry, meshes, solver
+    from pocketwind_gb300.batch import Batch
+    members, refs, own = [], [], []
+    for layout in layouts:
+        grid = geometry.voxelize(meshes.icosphere([n / 2.1 for n in layout], min(layout) / 5, 2), None, layout, False)
+        members.append(solver.GpuSolver.create(layout, grid, solver.SolverParams(tau0=0.56, u_in=0.05,
+                                                                                 precision=precision)))
+        refs.append(O.Wgsl32(*layout, 0.56, 0.05, grid.geometry, grid.boundary_cells))
+        own.append(O.Wgsl32(*layout, 0.56, 0.05, grid.geometry, grid.boundary_cells, storage=precision))
+    batch = Batch(members)
+    for n in counts:
+        batch.step(n, True)
+        for ref in refs + own:
+            for k in range(n):
+                ref.step(0.05, k + 1 == n)
+    for m, ref, o in zip(members, refs, own):
+        want = ref.populations()
+        assert _norm_err(m.populations(), want) <= (1e-5 if precision == "f32" else 2 * _norm_err(o.populations(), want))
+        assert not m.guard_unstable()
+    batch.destroy()
