@@ -23,7 +23,7 @@
 // memory, binary32 accumulators in tensor memory, issued by one thread and
 // read back by every thread for its own cells (tcgen05.ld); the update then
 // goes on with tau = tau0 + (tau_s - tau0) max(0, 1 + c).  The wall-link cells
-// and the floor layer run in the edge and floor kernels beside it with plain
+// and the floor layer run in blocks of their own in the same launch with plain
 // Smagorinsky and the reference's wall model, as in a step without the closure.
 // Free-slip faces (closure_step): one cell per thread over every cell, 128
 // cells per block, the same network on one tile; for the regularized operator
@@ -433,8 +433,8 @@ __global__ void __launch_bounds__(128, 4) closure_step(StepParams p, const uint3
 // runs as two M = 128 tiles, the threads' first cells and their second cells.
 // Every row of both parities runs here, the seam rows with their periodic
 // wrap as per-row offsets (SeamWrap); the wall-link cells and the floor layer
-// run in the edge and floor kernels beside it, with the reference's wall
-// model, as in a step without the closure.
+// run in blocks of their own, with the reference's wall model, as in a step
+// without the closure.
 struct TcPair {
   __align__(128) unsigned char img[kImgBytes];   // the network image
   // the layer-2 operands of the two tiles (128 x 32 bf16 each); the two
@@ -443,6 +443,7 @@ struct TcPair {
   __align__(128) unsigned char a2[2][128 * 64];
   __align__(8) uint64_t bar;                     // MMA completion
   uint32_t tmem;                                 // 64 TMEM columns: tile t's layer output at column 32 t
+  uint32_t next[2];                              // the block's next tile, by turns
   uint32_t failed;                               // a completion wait ran out
   __device__ __forceinline__ unsigned char *a1(int t) { return a2[0] + t * (128 * 32); }
 };
@@ -571,27 +572,74 @@ struct ClosureHook2 {
   }
 };
 
-// A persistent grid: each block sets up the network image and its TMEM
-// columns once, then walks tiles of 64 x 4 cells of one z-plane, tiles W apart
-// for W blocks.  Plain cells and EQ cells without wall links are stored, as in
-// aa_step_fast; every thread takes part in each tile's network.
+// The wall-link cells and the floor layer, as functions of their own (see pw_kernels_all.cu).
+template <int ST, int OP, bool ODD>
+__device__ __noinline__ void edge_role(const StepParams &p, const uint32_t *list, uint32_t count, uint32_t b) {
+  pwclosure::edge_block<ST, OP, true, ODD>(p, list, count, b, threadIdx.x + 32u * threadIdx.y);
+}
+template <int ST, int OP, bool ODD>
+__device__ __noinline__ void floor_role(const StepParams &p, uint32_t b, uint32_t runs) {
+  pwclosure::floor_thread<ST, OP, true, ODD>(p, (b % runs) * 64u + 2u * threadIdx.x,
+                                             1u + (b / runs) * 4u + threadIdx.y);
+}
+
+// One launch a step: the first blocks take the wall-link cells and the floor
+// layer, the others are a persistent grid: each sets up the network image and
+// its TMEM columns once, then walks tiles of 64 x 4 cells of one z-plane, tiles
+// W apart for W blocks.  Plain cells and EQ cells without wall links are stored,
+// as in aa_step_fast; every thread takes part in each tile's network.
 // Eight blocks per SM (64 registers; all 512 TMEM columns): measured 6%
 // faster than six (80 registers) and 9% faster than four.
+// A block's first tile is its own, the others it takes as it gets to them: blocks
+// that start after a side block, or whose cells take longer, take fewer.  The next
+// step's blocks set up their networks while this one's last ones run.  A step, before
+// (edge and floor kernels beside a static share of the tiles) and now: 96x48x48 FP16
+// 31.4 and 26.3 us, 128x64x64 FP32 37.6 and 36.0, 256x128x128 FP32 255 and 238,
+// 384x192x192 FP16 658 and 613 (64x32x32 as a 64-step graph 12.4, now 15.0).
 #ifndef PW_CLOSURE_PAIR_BLOCKS
 #define PW_CLOSURE_PAIR_BLOCKS 8
 #endif
 static_assert(PW_CLOSURE_PAIR_BLOCKS * 64 <= 512, "the blocks of an SM must fit its 512 TMEM columns");
+struct ClosureSide {
+  const uint32_t *list;
+  uint32_t count, edge, floor;
+  uint32_t *taken;  // tiles handed out beyond the blocks' first ones, this step's and the other parity's
+};
 template <int ST, int OP, bool ODD>
-__global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(StepParams p, const uint32_t *frag, const uint8_t *wall_dist,
-                                                        uint32_t runs, uint32_t row_blocks) {
+__global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(const __grid_constant__ StepParams p,
+                                                                            const uint32_t *frag,
+                                                                            const uint8_t *wall_dist, uint32_t runs,
+                                                                            uint32_t row_blocks, ClosureSide side) {
+  const uint32_t first = side.edge + side.floor;
+  if (blockIdx.x < first) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (blockIdx.x < side.edge) {
+      edge_role<ST, OP, ODD>(p, side.list, side.count, blockIdx.x);
+    } else {
+      if constexpr (ST != pw::STORE_F32) floor_role<ST, OP, ODD>(p, blockIdx.x - side.edge, runs);
+    }
+    return;
+  }
   using S = pw::Store<ST>;
   using T = typename S::T;
   __shared__ TcPair sh;
   tc_setup(sh, frag);
-  uint32_t phase = 0;
+  // the next step's blocks may come once every block here has its TMEM columns
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const bool leader = (threadIdx.x | threadIdx.y) == 0u;
+  if (leader && blockIdx.x == first) {
+    if (p.clear_status) *p.status = 0u;
+    side.taken[ODD ? 0 : 1] = 0u;  // the next step's
+  }
+  uint32_t phase = 0, turn = 0;
   T *f = reinterpret_cast<T *>(p.f);
   const uint32_t tiles = runs * row_blocks * p.nz;
-  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  uint32_t next = 0;
+  for (uint32_t tile = blockIdx.x - first; tile < tiles; tile = next) {
+    // the tile after this one; every thread reads it behind the network's barriers
+    if (leader) sh.next[turn & 1u] = gridDim.x - first + atomicAdd(&side.taken[ODD ? 1 : 0], 1u);
     const uint32_t run = tile % runs, rest = tile / runs;
     const uint32_t x = run * 64u + threadIdx.x, y = (rest % row_blocks) * 4u + threadIdx.y, z = rest / row_blocks;
     const bool row_in = y < p.ny;
@@ -642,6 +690,8 @@ __global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(Ste
     float2 rho, vx, vy, vz;
     const float2 om = pwclosure::update_fast2<OP, true, ClosureHook2>(
         p, g, rho, vx, vy, vz, S::kScale, S::kInvScale, eq, eux, euy, euz, ClosureHook2{&sh, &phase, wall, live});
+    next = sh.next[turn & 1u];
+    turn++;
     if (!ok) continue;
     if (ST != pw::STORE_F32) {
       // a non-finite state is stored as NaN, as the reference's GPUs store it
@@ -1218,39 +1268,34 @@ void launch_closure_step(const StepParams &p, int storage, int op, bool odd, dim
 
 template <int ST, int OP, bool ODD>
 static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const uint8_t *wall, const uint32_t *list,
-                               uint32_t count, cudaStream_t s, cudaStream_t t) {
-  // the grid is the blocks that fit at once: the launch bound's count per SM
-  // (registers; 20 KB of shared memory and 64 TMEM columns a block leave room
-  // for more).  No occupancy query: the first step may run under stream capture.
-  const int blocks_per_sm = PW_CLOSURE_PAIR_BLOCKS;
-  // the floor layer and the wall-link cells beside the plain cells
-  if constexpr (ST != pw::STORE_F32) {
-    if (p.floor_rows && p.ny >= 3u) {
-      const dim3 grid((p.nx + 2 * pwclosure::BX - 1) / (2 * pwclosure::BX), (p.ny - 2u + pwclosure::BY - 1u) / pwclosure::BY);
-      pwclosure::aa_step_floor<ST, OP, true, ODD><<<grid, dim3(pwclosure::BX, pwclosure::BY), 0, t>>>(p);
-    }
-  }
-  if (count)
-    pwclosure::aa_step_edges<ST, OP, true, ODD>
-        <<<(count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, pwclosure::NTHREADS, 0, t>>>(p, list, count);
+                               uint32_t count, uint32_t *taken, cudaStream_t s) {
+  // the blocks that fit at once: the launch bound's count per SM (registers; 20 KB of
+  // shared memory and 64 TMEM columns a block leave room for more)
+  const uint32_t fit = (uint32_t)PW_CLOSURE_PAIR_BLOCKS * (uint32_t)sm_count();
   const uint32_t runs = (p.nx + 63u) / 64u, row_blocks = (p.ny + 3u) / 4u;
   const uint32_t tiles = runs * row_blocks * p.nz;
-  const unsigned g = (unsigned)std::min<uint32_t>(tiles, (uint32_t)blocks_per_sm * (uint32_t)sm_count());
-  closure_pairs<ST, OP, ODD><<<g, dim3(32, 4), 0, s>>>(p, frag, wall, runs, row_blocks);
+  ClosureSide side{list, count, (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, 0u, taken};
+  if (ST != pw::STORE_F32 && p.floor_rows && p.ny >= 3u) side.floor = runs * ((p.ny - 2u + 3u) / 4u);
+  const uint32_t first = side.edge + side.floor, walk = std::min(tiles, fit);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(first + walk);
+  cfg.blockDim = dim3(32, 4);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, closure_pairs<ST, OP, ODD>, p, frag, wall, runs, row_blocks, side);
 }
 
 void launch_closure_pairs(const StepParams &p, int storage, int op, bool odd, const uint32_t *frag,
-                          const uint8_t *wall, const uint32_t *list, uint32_t count, cudaStream_t s,
-                          const pwfast::SideStream *side) {
-  cudaStream_t t = side ? side->stream : s;
-  if (side) {
-    cudaEventRecord(side->fork, s);
-    cudaStreamWaitEvent(t, side->fork, 0);
-  }
-#define PW_CLP(ST, OPV)                                                             \
-  do {                                                                              \
-    if (odd) closure_pairs_step<ST, OPV, true>(p, frag, wall, list, count, s, t);   \
-    else closure_pairs_step<ST, OPV, false>(p, frag, wall, list, count, s, t);      \
+                          const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken,
+                          cudaStream_t s) {
+#define PW_CLP(ST, OPV)                                                          \
+  do {                                                                           \
+    if (odd) closure_pairs_step<ST, OPV, true>(p, frag, wall, list, count, taken, s);   \
+    else closure_pairs_step<ST, OPV, false>(p, frag, wall, list, count, taken, s);      \
   } while (0)
   if (op == pw::OP_REG) {
     if (storage == pw::STORE_F16) PW_CLP(pw::STORE_F16, pw::OP_REG);
@@ -1262,10 +1307,6 @@ void launch_closure_pairs(const StepParams &p, int storage, int op, bool odd, co
     else PW_CLP(pw::STORE_F32, pw::OP_TRT);
   }
 #undef PW_CLP
-  if (side) {
-    cudaEventRecord(side->join, t);
-    cudaStreamWaitEvent(s, side->join, 0);
-  }
 }
 
 int wall_distance_of(const uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *out, cudaStream_t s) {

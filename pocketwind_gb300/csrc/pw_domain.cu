@@ -213,6 +213,7 @@ struct pw_domain {
   uint32_t edge_own = 0;          // the list's head that a domain's own step runs (all but its floor cells)
   dim3 plain_grid;                // the cell grid, or empty when no plain position exists
   const uint32_t *closure_frag = nullptr;  // attached learned closure (its weight fragments)
+  uint32_t *tiles_taken = nullptr;  // the closure step's tile counters (two, by parity)
   uint8_t *wall_dist = nullptr;   // cells to the nearest wall, for the closure's inputs
   bool interp = false;            // interpolated (Bouzidi) walls
   uint32_t *qoff = nullptr;       // per cell: first wall-link fraction (interpolated walls)
@@ -285,13 +286,16 @@ pw::StepParams params_for(const pw_domain *d, uint64_t step, float u_in, int wri
   return p;
 }
 
+// Whether a step is one launch (the split step in that form, the closure's cell pairs).
+bool single_launch(const pw_domain *d) { return d->split && (d->one_launch || d->closure_frag); }
+
 // Queue step number `step` (1-based) with the given inlet speed.  The guard's flag of a
 // macro step starts at zero: a step of one launch before it in the same call clears it
 // (before_macro, then cleared), without a memset between the two.
 void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool before_macro = false,
                   bool cleared = false, bool early = true) {
   pw::StepParams p = params_for(d, step, u_in, write_macro);
-  const bool one = d->one_launch && d->split && !d->closure_frag;
+  const bool one = single_launch(d);
   p.clear_status = one && before_macro ? 1 : 0;
   if (write_macro && !(one && cleared)) cudaMemsetAsync(d->status_dev, 0, 4, d->stream);
   bool odd = (step & 1) != 0;
@@ -305,7 +309,7 @@ void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool
     pwstrict::launch_step(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->grid, d->stream);
   else if (d->closure_frag && d->split)
     pwclosure_host::launch_closure_pairs(p, d->desc.storage, d->desc.op, odd, d->closure_frag, d->wall_dist, d->edges,
-                                         d->edge_own, d->stream, &d->side);
+                                         d->edge_own, d->tiles_taken, d->stream);
   else if (d->closure_frag)
     pwclosure_host::launch_closure_step(p, d->desc.storage, d->desc.op, odd, d->grid, d->closure_frag, d->wall_dist,
                                         d->stream);
@@ -342,6 +346,7 @@ void interp_state(pw_domain *d, uint64_t steps, int refresh) {
 }
 
 int launch_init(pw_domain *d) {
+  PW_TRY(cudaMemsetAsync(d->tiles_taken, 0, 2 * sizeof(uint32_t), d->stream));
   float u0 = d->desc.ramp_steps > 0 ? 0.0f : d->u_in;
   // every cell's slots are written below (a wall's with zeros); what lies between
   // the planes' cells and their stride is cleared here
@@ -628,6 +633,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   a.want((void **)&d->plane[0], plane_n * sizeof(float4));
   a.want((void **)&d->plane[1], plane_n * sizeof(float4));
   a.want((void **)&d->status_dev, 16);
+  a.want((void **)&d->tiles_taken, 2 * sizeof(uint32_t));
   a.want((void **)&d->totals_dev, 4 * sizeof(double));
   if (e == cudaSuccess) e = a.alloc(&d->arena);
   if (e == cudaSuccess) {
@@ -727,9 +733,7 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
   // the 128x64x64 FP32 vehicle's step took as long), and a split step of more than a
   // million cells is faster without (its side kernels lose their head start in a graph:
   // 192x96x96 FP16 45.9 us a step against 37.9; 128x64x64 24.0 against 28.9).
-  const bool one_launch = d->one_launch && !d->closure_frag;
-  const bool split = d->split && !d->closure_frag;
-  const bool use_graphs = !one_launch && d->cells <= (size_t)(split ? 1 : 8) << 20;
+  const bool use_graphs = !single_launch(d) && d->cells <= (size_t)(d->split ? 1 : 8) << 20;
   while (use_graphs && count - k >= (uint64_t)kGraphChunk) {
     int macro_last = write_macro_on_last && (count - k == (uint64_t)kGraphChunk);
     cudaGraphExec_t g = graph_for(d, (int)((d->steps + 1) & 1), macro_last);
