@@ -573,11 +573,11 @@ struct ClosureHook2 {
 };
 
 // The wall-link cells and the floor layer, as functions of their own (see pw_kernels_all.cu).
-template <int ST, int OP, bool ODD>
+template <int ST, int OP, bool ODD, int BLOCKS>
 __device__ __noinline__ void edge_role(const StepParams &p, const uint32_t *list, uint32_t count, uint32_t b) {
   pwclosure::edge_block<ST, OP, true, ODD>(p, list, count, b, threadIdx.x + 32u * threadIdx.y);
 }
-template <int ST, int OP, bool ODD>
+template <int ST, int OP, bool ODD, int BLOCKS>
 __device__ __noinline__ void floor_role(const StepParams &p, uint32_t b, uint32_t runs) {
   pwclosure::floor_thread<ST, OP, true, ODD>(p, (b % runs) * 64u + 2u * threadIdx.x,
                                              1u + (b / runs) * 4u + threadIdx.y);
@@ -594,19 +594,24 @@ __device__ __noinline__ void floor_role(const StepParams &p, uint32_t b, uint32_
 // that start after a side block, or whose cells take longer, take fewer.  The next
 // step's blocks set up their networks while this one's last ones run.  A step, before
 // (edge and floor kernels beside a static share of the tiles) and now: 96x48x48 FP16
-// 31.4 and 26.3 us, 128x64x64 FP32 37.6 and 36.0, 256x128x128 FP32 255 and 238,
-// 384x192x192 FP16 658 and 613 (64x32x32 as a 64-step graph 12.4, now 15.0).
+// 31.4 and 26.5 us, 128x64x64 FP32 37.3 and 36.2, 256x128x128 FP32 255 and 238,
+// 384x192x192 FP16 658 and 603.
+// A step whose blocks all find a place at four per SM runs in the form with their 128
+// registers: its time is one tile's and one wall-link cell's, whose spilled registers
+// count then (64x32x32 FP32 15.3 and 13.4 us with 64 and 128 registers, FP16 18.2 and
+// 14.9; separate kernels 15.9 and 23.8 in short calls, 12.3 and 18.9 in captured ones).
 #ifndef PW_CLOSURE_PAIR_BLOCKS
 #define PW_CLOSURE_PAIR_BLOCKS 8
 #endif
+#define PW_CLOSURE_FEW_BLOCKS 4
 static_assert(PW_CLOSURE_PAIR_BLOCKS * 64 <= 512, "the blocks of an SM must fit its 512 TMEM columns");
 struct ClosureSide {
   const uint32_t *list;
   uint32_t count, edge, floor;
-  uint32_t *taken;  // tiles handed out beyond the blocks' first ones, this step's and the other parity's
+  uint32_t *taken;  // tiles handed out beyond the blocks' first ones; zero between steps
 };
-template <int ST, int OP, bool ODD>
-__global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(const __grid_constant__ StepParams p,
+template <int ST, int OP, bool ODD, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) closure_pairs(const __grid_constant__ StepParams p,
                                                                             const uint32_t *frag,
                                                                             const uint8_t *wall_dist, uint32_t runs,
                                                                             uint32_t row_blocks, ClosureSide side) {
@@ -615,9 +620,9 @@ __global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(con
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (blockIdx.x < side.edge) {
-      edge_role<ST, OP, ODD>(p, side.list, side.count, blockIdx.x);
+      edge_role<ST, OP, ODD, BLOCKS>(p, side.list, side.count, blockIdx.x);
     } else {
-      if constexpr (ST != pw::STORE_F32) floor_role<ST, OP, ODD>(p, blockIdx.x - side.edge, runs);
+      if constexpr (ST != pw::STORE_F32) floor_role<ST, OP, ODD, BLOCKS>(p, blockIdx.x - side.edge, runs);
     }
     return;
   }
@@ -629,17 +634,18 @@ __global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(con
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const bool leader = (threadIdx.x | threadIdx.y) == 0u;
-  if (leader && blockIdx.x == first) {
-    if (p.clear_status) *p.status = 0u;
-    side.taken[ODD ? 0 : 1] = 0u;  // the next step's
-  }
+  if (leader && blockIdx.x == first && p.clear_status) *p.status = 0u;
   uint32_t phase = 0, turn = 0;
   T *f = reinterpret_cast<T *>(p.f);
   const uint32_t tiles = runs * row_blocks * p.nz;
-  uint32_t next = 0;
+  const bool more = gridDim.x - first < tiles;  // tiles beyond the blocks' first ones
+  uint32_t next = tiles;
   for (uint32_t tile = blockIdx.x - first; tile < tiles; tile = next) {
-    // the tile after this one; every thread reads it behind the network's barriers
-    if (leader) sh.next[turn & 1u] = gridDim.x - first + atomicAdd(&side.taken[ODD ? 1 : 0], 1u);
+    // the tile after this one, stored once this one's loads are under way; every thread
+    // reads it behind the network's barriers.  One is asked for per tile taken, so the
+    // count wraps to zero with the step's last.
+    uint32_t got = 0;
+    if (more && leader) got = atomicInc(side.taken, tiles - 1u);
     const uint32_t run = tile % runs, rest = tile / runs;
     const uint32_t x = run * 64u + threadIdx.x, y = (rest % row_blocks) * 4u + threadIdx.y, z = rest / row_blocks;
     const bool row_in = y < p.ny;
@@ -674,6 +680,7 @@ __global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(con
 #pragma unroll
       for (int i = 0; i < 19; i++) g[i] = make_float2(0.0f, 0.0f);
     }
+    if (more && leader) sh.next[turn & 1u] = gridDim.x - first + got;
     float2 eux = pwclosure::f2(p.u_in), euy = pwclosure::f2(0.f), euz = pwclosure::f2(0.f);
     if (eq) {
       const uint32_t row = y + p.ny * z;
@@ -690,7 +697,7 @@ __global__ void __launch_bounds__(128, PW_CLOSURE_PAIR_BLOCKS) closure_pairs(con
     float2 rho, vx, vy, vz;
     const float2 om = pwclosure::update_fast2<OP, true, ClosureHook2>(
         p, g, rho, vx, vy, vz, S::kScale, S::kInvScale, eq, eux, euy, euz, ClosureHook2{&sh, &phase, wall, live});
-    next = sh.next[turn & 1u];
+    if (more) next = sh.next[turn & 1u];
     turn++;
     if (!ok) continue;
     if (ST != pw::STORE_F32) {
@@ -1266,36 +1273,43 @@ void launch_closure_step(const StepParams &p, int storage, int op, bool odd, dim
 #undef PW_CL_LAUNCH
 }
 
-template <int ST, int OP, bool ODD>
-static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const uint8_t *wall, const uint32_t *list,
-                               uint32_t count, uint32_t *taken, cudaStream_t s) {
+template <int ST, int OP, bool ODD, int BLOCKS>
+static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const uint8_t *wall, uint32_t runs,
+                               uint32_t row_blocks, const ClosureSide &side, bool early, cudaStream_t s) {
   // the blocks that fit at once: the launch bound's count per SM (registers; 20 KB of
   // shared memory and 64 TMEM columns a block leave room for more)
-  const uint32_t fit = (uint32_t)PW_CLOSURE_PAIR_BLOCKS * (uint32_t)sm_count();
-  const uint32_t runs = (p.nx + 63u) / 64u, row_blocks = (p.ny + 3u) / 4u;
-  const uint32_t tiles = runs * row_blocks * p.nz;
-  ClosureSide side{list, count, (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, 0u, taken};
-  if (ST != pw::STORE_F32 && p.floor_rows && p.ny >= 3u) side.floor = runs * ((p.ny - 2u + 3u) / 4u);
-  const uint32_t first = side.edge + side.floor, walk = std::min(tiles, fit);
+  const uint32_t tiles = runs * row_blocks * p.nz, walk = std::min(tiles, (uint32_t)BLOCKS * (uint32_t)sm_count());
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(first + walk);
+  cfg.gridDim = dim3(side.edge + side.floor + walk);
   cfg.blockDim = dim3(32, 4);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, closure_pairs<ST, OP, ODD>, p, frag, wall, runs, row_blocks, side);
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, closure_pairs<ST, OP, ODD, BLOCKS>, p, frag, wall, runs, row_blocks, side);
+}
+
+template <int ST, int OP, bool ODD>
+static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const uint8_t *wall, const uint32_t *list,
+                               uint32_t count, uint32_t *taken, bool early, cudaStream_t s) {
+  const uint32_t runs = (p.nx + 63u) / 64u, row_blocks = (p.ny + 3u) / 4u;
+  ClosureSide side{list, count, (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, 0u, taken};
+  if (ST != pw::STORE_F32 && p.floor_rows && p.ny >= 3u) side.floor = runs * ((p.ny - 2u + 3u) / 4u);
+  if ((uint64_t)runs * row_blocks * p.nz + side.edge + side.floor <= (uint64_t)PW_CLOSURE_FEW_BLOCKS * sm_count())
+    closure_pairs_step<ST, OP, ODD, PW_CLOSURE_FEW_BLOCKS>(p, frag, wall, runs, row_blocks, side, early, s);
+  else
+    closure_pairs_step<ST, OP, ODD, PW_CLOSURE_PAIR_BLOCKS>(p, frag, wall, runs, row_blocks, side, early, s);
 }
 
 void launch_closure_pairs(const StepParams &p, int storage, int op, bool odd, const uint32_t *frag,
                           const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken,
-                          cudaStream_t s) {
+                          bool early, cudaStream_t s) {
 #define PW_CLP(ST, OPV)                                                          \
   do {                                                                           \
-    if (odd) closure_pairs_step<ST, OPV, true>(p, frag, wall, list, count, taken, s);   \
-    else closure_pairs_step<ST, OPV, false>(p, frag, wall, list, count, taken, s);      \
+    if (odd) closure_pairs_step<ST, OPV, true>(p, frag, wall, list, count, taken, early, s);   \
+    else closure_pairs_step<ST, OPV, false>(p, frag, wall, list, count, taken, early, s);      \
   } while (0)
   if (op == pw::OP_REG) {
     if (storage == pw::STORE_F16) PW_CLP(pw::STORE_F16, pw::OP_REG);

@@ -213,7 +213,7 @@ struct pw_domain {
   uint32_t edge_own = 0;          // the list's head that a domain's own step runs (all but its floor cells)
   dim3 plain_grid;                // the cell grid, or empty when no plain position exists
   const uint32_t *closure_frag = nullptr;  // attached learned closure (its weight fragments)
-  uint32_t *tiles_taken = nullptr;  // the closure step's tile counters (two, by parity)
+  uint32_t *tiles_taken = nullptr;  // the closure step's tile counter, zero between steps
   uint8_t *wall_dist = nullptr;   // cells to the nearest wall, for the closure's inputs
   bool interp = false;            // interpolated (Bouzidi) walls
   uint32_t *qoff = nullptr;       // per cell: first wall-link fraction (interpolated walls)
@@ -309,7 +309,7 @@ void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool
     pwstrict::launch_step(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->grid, d->stream);
   else if (d->closure_frag && d->split)
     pwclosure_host::launch_closure_pairs(p, d->desc.storage, d->desc.op, odd, d->closure_frag, d->wall_dist, d->edges,
-                                         d->edge_own, d->tiles_taken, d->stream);
+                                         d->edge_own, d->tiles_taken, early, d->stream);
   else if (d->closure_frag)
     pwclosure_host::launch_closure_step(p, d->desc.storage, d->desc.op, odd, d->grid, d->closure_frag, d->wall_dist,
                                         d->stream);
@@ -346,7 +346,7 @@ void interp_state(pw_domain *d, uint64_t steps, int refresh) {
 }
 
 int launch_init(pw_domain *d) {
-  PW_TRY(cudaMemsetAsync(d->tiles_taken, 0, 2 * sizeof(uint32_t), d->stream));
+  PW_TRY(cudaMemsetAsync(d->tiles_taken, 0, sizeof(uint32_t), d->stream));
   float u0 = d->desc.ramp_steps > 0 ? 0.0f : d->u_in;
   // every cell's slots are written below (a wall's with zeros); what lies between
   // the planes' cells and their stride is cleared here
@@ -437,7 +437,8 @@ cudaGraphExec_t graph_for(pw_domain *d, int start_parity, int macro_last) {
   if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
     for (int k = 0; k < kGraphChunk; k++) {
       uint64_t step = (uint64_t)start_parity + (uint64_t)k;  // only the parity matters
-      enqueue_step(d, step == 0 ? 2 : step, d->u_in, macro_last && k == kGraphChunk - 1);
+      enqueue_step(d, step == 0 ? 2 : step, d->u_in, macro_last && k == kGraphChunk - 1, false, false,
+                   false);
     }
     if (cudaStreamEndCapture(cap, &graph) == cudaSuccess && graph) {
       if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) exec = nullptr;
@@ -633,7 +634,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   a.want((void **)&d->plane[0], plane_n * sizeof(float4));
   a.want((void **)&d->plane[1], plane_n * sizeof(float4));
   a.want((void **)&d->status_dev, 16);
-  a.want((void **)&d->tiles_taken, 2 * sizeof(uint32_t));
+  a.want((void **)&d->tiles_taken, sizeof(uint32_t));
   a.want((void **)&d->totals_dev, 4 * sizeof(double));
   if (e == cudaSuccess) e = a.alloc(&d->arena);
   if (e == cudaSuccess) {

@@ -77,10 +77,11 @@ void launch_closure_step(const pw::StepParams &p, int storage, int op, bool odd,
                          const uint8_t *wall, cudaStream_t s);
 // The same step for periodic faces in the cell-pair form, one launch: every row's
 // plain cells two per thread with the network on the block's two 128-cell tiles, and
-// the listed edge cells and the floor layer in blocks of their own; taken: two counters,
-// zero before the first step.
+// the listed edge cells and the floor layer in blocks of their own; taken: a counter that
+// is zero between steps; early: the step may start while the one before it ends.
 void launch_closure_pairs(const pw::StepParams &p, int storage, int op, bool odd, const uint32_t *frag,
-                          const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken, cudaStream_t s);
+                          const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken, bool early,
+                          cudaStream_t s);
 int wall_distance_of(const uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *out, cudaStream_t s);
 const uint32_t *fragments(const pw_closure *c);
 }

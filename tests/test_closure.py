@@ -272,6 +272,36 @@ def test_closure_step_is_deterministic():
 
 
 @pytest_gpu
+@pytest.mark.parametrize("nx", [32, 128])
+def test_closure_step_hands_out_every_tile(nx):
+    """Tiles handed out beyond the blocks' first ones (128) and none (32): steps one by
+    one and in one call, and steps from a state loaded at once and after an odd number
+    of further steps, give the same stored codes bit for bit."""
+    from pocketwind_gb300 import cases, solver
+    v = cases.vehicle_case(nx)
+    net = _closure(_rand_params(9))
+
+    def codes(single, more=None):
+        s = solver.GpuSolver.create(v.layout, v.grid(), solver.SolverParams(tau0=v.tau0, u_in=0.05, les=True,
+                                                                             operator="reg", precision="f16"))
+        net.attach(s)
+        s.step(2, True)
+        if more is not None:
+            blob = s.save_checkpoint()
+            s.step(more)
+            s.load_checkpoint(blob)
+        for n in [1] * 71 if single else [71]:
+            s.step(n)
+        out = s.populations_raw().view(np.uint8).copy()
+        s.destroy()
+        return out
+
+    assert np.array_equal(codes(True), codes(False))
+    assert np.array_equal(codes(False, more=0), codes(False, more=1))
+    net.destroy()
+
+
+@pytest_gpu
 def test_trained_closure_beats_smagorinsky_on_held_out_data():
     """What the network gains over the method without it: after training on
     filtered fine-grid samples its a-priori error on held-out samples is below
