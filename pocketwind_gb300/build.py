@@ -26,6 +26,8 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "pw_kernels_fast.cu": [],
     "pw_kernels_all.cu": [],
+    "pw_kernels_all_f16.cu": [],
+    "pw_kernels_all_bf16.cu": [],
     "pw_kernels_strict.cu": ["-fmad=false"],
     "pw_geometry.cu": ["-fmad=false"],
     "pw_tracers.cu": ["-fmad=false"],
@@ -34,7 +36,8 @@ UNITS = {
     "pw_batch.cu": [],
     "pw_closure.cu": [],
 }
-HEADERS = ["pw_common.cuh", "pw_lbm.cuh", "pw_lbm_tile.cuh", "pw_launch.h", "pw_internal.h", "pw_closure.cuh"]
+HEADERS = ["pw_common.cuh", "pw_lbm.cuh", "pw_lbm_tile.cuh", "pw_step_all.cuh", "pw_launch.h", "pw_internal.h",
+           "pw_closure.cuh"]
 
 
 def nvcc() -> str:

@@ -572,7 +572,7 @@ struct ClosureHook2 {
   }
 };
 
-// The wall-link cells and the floor layer, as functions of their own (see pw_kernels_all.cu).
+// The wall-link cells and the floor layer, as functions of their own (see pw_step_all.cuh).
 template <int ST, int OP, bool ODD, int BLOCKS>
 __device__ __noinline__ void edge_role(const StepParams &p, const uint32_t *list, uint32_t count, uint32_t b) {
   pwclosure::edge_block<ST, OP, true, ODD>(p, list, count, b, threadIdx.x + 32u * threadIdx.y);

@@ -58,7 +58,7 @@ void launch_refresh_edges(const pw::StepParams &p, int odd_layout, int storage, 
                           uint32_t count, cudaStream_t s);
 }
 PW_DECLARE_LAUNCHERS(pwstrict)
-// The same split step in one launch, blocks by role (pw_kernels_all.cu).
+// The same split step in one launch, blocks by role (pw_step_all.cuh).
 namespace pwall {
 bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int les, uint32_t slip);
 // early: the launch may start while the step before it on the stream still runs (its

@@ -633,3 +633,34 @@ def test_step_at_small_and_ragged_sizes(layout, precision, floor):
     assert norm_err(s.populations(), ref.populations()) <= tol
     assert norm_err(s.macros().reshape(-1), ref.macros().reshape(-1)) <= tol
     s.destroy()
+
+
+# the lines between the one-launch step's forms by plain blocks per SM (152): 4 below 16,
+# 6 with LES below 32 (binary32) or 48 (16-bit pairs), one block a plane here (odd steps
+# leave two planes out, so both parities of one size may take different forms)
+@pytest.mark.parametrize("periods", [101, 102, 202, 203, 304, 305])
+def test_step_between_block_forms_repeats_a_period(periods):
+    """A binary32 LES domain whose cells repeat every 24 planes: after 9 steps every period
+    beyond the reach of the z faces' rows has the bits of the middle one of three (a domain
+    of the first form)."""
+    r = np.random.default_rng(24)
+    kinds = np.where(r.random((24, 4, 4)) < 0.1, SOLID, FLUID)
+    kinds[:, :, 0] = kinds[:, :, -1] = EQ
+    got = []
+    for n in (3, periods):
+        layout = (4, 4, 24 * n)
+        geometry, boundary = grid_from_kinds(layout, np.tile(kinds, (n, 1, 1)).reshape(-1))
+        s = make_solver(geometry, boundary, layout, les=True)
+        s.step(1, True)
+        s.step(8, True)
+        got.append((s.populations().reshape(19, n, -1), s.macros().reshape(n, -1)))
+        s.destroy()
+    assert np.array_equal(got[1][0][:, 1:-1], np.repeat(got[0][0][:, 1:2], periods - 2, axis=1))
+    assert np.array_equal(got[1][1][1:-1], np.repeat(got[0][1][1:2], periods - 2, axis=0))
+
+
+@pytest.mark.parametrize("nx,nz", [(4, 2431), (4, 2433), (5, 2431), (5, 2433)])
+@pytest.mark.parametrize("precision", ["f32", "f16"])
+def test_step_between_block_forms(nx, nz, precision):
+    """As test_step_at_small_and_ragged_sizes, on both sides of the first line."""
+    test_step_at_small_and_ragged_sizes((nx, 4, nz), precision, False)
