@@ -253,7 +253,9 @@ __device__ __forceinline__ float update_fast(const StepParams &p, float *g, floa
   vx = jx * vs;
   vy = jy * vs;
   vz = jz * vs;
-  const float uu = vx * vx + vy * vy + vz * vz;
+  // (fused as written: left to the compiler, the choice changed with the kernel around
+  // it, and the stored 16-bit codes with it)
+  const float uu = __fmaf_rn(vz, vz, __fmaf_rn(vx, vx, vy * vy));
   const float K = rd - 1.5f * rho * uu;  // rd + rho(-1.5 uu): the cu-free part of the equilibrium
   float om_p = p.omega_plus, om_m = p.omega_minus;
   float pxx = 0.f, pyy = 0.f, pzz = 0.f, pxy = 0.f, pxz = 0.f, pyz = 0.f;
