@@ -683,7 +683,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   int rc = PW_OK;
   if (!d->tiled && !desc->strict) {
     d->split = true;
-    d->one_launch = pwall::step_all_supported(d->nx, d->ny, d->nz, desc->storage, desc->les, d->slip);
+    d->one_launch = pwall::step_all_supported(d->nx, d->ny, d->nz, desc->storage, desc->op, desc->les, d->slip);
     rc = build_edge_list(d);
   }
   if (rc == PW_OK) rc = launch_init(d);

@@ -12,13 +12,16 @@ extern template void launch_storage<STORE_BF16>(const StepParams &, int, int, bo
 // at 64^2 x 128 23.4 us before and 15.2 now, at 256^2 x 512 795 and 794).  16-bit cell
 // pairs: up to 8 M cells (4.2 M: 73.9 us before, 71.5 now; 14 M: 222.8 and 224.9, where
 // the side kernels' registers no longer pay), and not beside reflecting seam rows, which
-// take one cell a thread.  16-bit storage with nx odd: any size without LES (203x101x67:
-// 35.0 and 24.4, 399x200x200: 308 and 266); with LES the seam rows' rounding depends on the kernel around them.
+// take one cell a thread.  16-bit storage with nx odd: any size (203x101x67 without LES
+// 35.0 and 24.4, 399x200x200 308 and 266; FP16 REG with LES 97x48x48 25.5 and 16.1,
+// 203x101x101 48.4 and 37.4, 399x199x199 298 and 266; free-slip BF16 97x48x48 59 and
+// 17), but FP16 TRT with LES: the compiler rounds that seam's rows differently in this
+// kernel than in aa_step_seam, in the last bit, and the stored codes with it.
 // The side blocks take at most five slices a plane, and a grid has 65,535.
-bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int les, uint32_t slip) {
+bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int op, int les, uint32_t slip) {
   if (nx < 3u || ny < 3u || nz < 3u || nz > 8192u) return false;
   if (storage == STORE_F32) return true;
-  if (nx & 1u) return !les && (uint64_t)nx * ny < (1ull << 31) - 2048u;
+  if (nx & 1u) return !(les && op == OP_TRT && storage == STORE_F16) && (uint64_t)nx * ny < (1ull << 31) - 2048u;
   return slip == 0u && (uint64_t)nx * ny * nz <= 8ull << 20;
 }
 

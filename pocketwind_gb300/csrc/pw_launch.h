@@ -60,7 +60,7 @@ void launch_refresh_edges(const pw::StepParams &p, int odd_layout, int storage, 
 PW_DECLARE_LAUNCHERS(pwstrict)
 // The same split step in one launch, blocks by role (pw_step_all.cuh).
 namespace pwall {
-bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int les, uint32_t slip);
+bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int op, int les, uint32_t slip);
 // early: the launch may start while the step before it on the stream still runs (its
 // blocks wait, holding their places: not for domains stepped side by side).
 void launch_step_all(const pw::StepParams &p, int storage, int op, int les, bool odd, const uint32_t *list,

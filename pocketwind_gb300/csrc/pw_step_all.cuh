@@ -162,10 +162,17 @@ void launch3(const StepParams &p, int op, bool odd, const uint32_t *list, uint32
   else launch4<ST, OP_TRT, LES, FORM>(p, odd, list, count, s, early);
 }
 
+// The pairs of a plane with LES, the operators that step_all_supported admits.
+template <int ST, Plain FORM>
+void launch_linear_les(const StepParams &p, int op, bool odd, const uint32_t *list, uint32_t count, cudaStream_t s,
+                       bool early) {
+  if constexpr (ST == STORE_F16) launch4<ST, OP_REG, true, FORM>(p, odd, list, count, s, early);
+  else launch3<ST, true, FORM>(p, op, odd, list, count, s, early);
+}
+
 }  // namespace
 
-// The step of one storage type; 16-bit: pairs of a row, or of a plane with nx odd
-// (without LES).
+// The step of one storage type; 16-bit: pairs of a row, or of a plane with nx odd.
 template <int ST>
 void launch_storage(const StepParams &p, int op, int les, bool odd, const uint32_t *list, uint32_t count,
                     cudaStream_t s, bool early) {
@@ -176,9 +183,11 @@ void launch_storage(const StepParams &p, int op, int les, bool odd, const uint32
     if (les) launch3<ST, true, PAIRS>(p, op, odd, list, count, s, early);
     else launch3<ST, false, PAIRS>(p, op, odd, list, count, s, early);
   } else if (p.ny & 1u) {
-    launch3<ST, false, LINEAR_NY_ODD>(p, op, odd, list, count, s, early);
+    if (!les) launch3<ST, false, LINEAR_NY_ODD>(p, op, odd, list, count, s, early);
+    else launch_linear_les<ST, LINEAR_NY_ODD>(p, op, odd, list, count, s, early);
   } else {
-    launch3<ST, false, LINEAR>(p, op, odd, list, count, s, early);
+    if (!les) launch3<ST, false, LINEAR>(p, op, odd, list, count, s, early);
+    else launch_linear_les<ST, LINEAR>(p, op, odd, list, count, s, early);
   }
 }
 

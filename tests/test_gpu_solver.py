@@ -664,3 +664,27 @@ def test_step_between_block_forms_repeats_a_period(periods):
 def test_step_between_block_forms(nx, nz, precision):
     """As test_step_at_small_and_ragged_sizes, on both sides of the first line."""
     test_step_at_small_and_ragged_sizes((nx, 4, nz), precision, False)
+
+
+@pytest.mark.parametrize("precision", ["f16", "bf16"])
+@pytest.mark.parametrize("op", ["trt", "reg"])
+@pytest.mark.parametrize("layout", [(49, 24, 24), (47, 25, 23)])
+def test_odd_rows_with_les_within_reference_rounding_noise(layout, op, precision):
+    """nx odd, 16-bit storage, LES (pairs over a plane's cells, ny even and odd; FP16 TRT in
+    kernels of its own): the bound of test_fast_16bit_within_reference_rounding_noise."""
+    from pocketwind_gb300 import meshes
+    G, S = _pw()
+    grid = O.voxelize(meshes.icosphere((12.3, 11.62, 12.41), 4, 3).positions, None, layout, False,
+                      link_fractions=False)
+    fast = make_solver(grid.geometry, grid.boundary_cells, layout, tau0=0.56, u_in=0.05, les=True, op=op,
+                       precision=precision)
+    ref32, ref16 = (O.Wgsl32(*layout, 0.56, 0.05, grid.geometry, grid.boundary_cells, les=True, op=op, storage=st)
+                    for st in ("f32", precision))
+    fast.step(16, True)
+    for k in range(16):
+        ref32.step(0.05, k == 15)
+        ref16.step(0.05, k == 15)
+    want = ref32.populations()
+    err, ref_err = norm_err(fast.populations(), want), norm_err(ref16.populations(), want)
+    assert np.isfinite(err) and err <= 2 * ref_err, (err, ref_err)
+    fast.destroy()
