@@ -45,8 +45,8 @@ __device__ __noinline__ void seam_role(const StepParams &p, uint32_t b) {
 // cells: about 9 us) and by launches: three or four of them, forked to a second
 // stream and joined, against one here, whose successor is launched while it runs
 // (griddepcontrol).  A step in a run of eight, before and now: 64x32x32 20.4 and
-// 12.3 us, 128x64x64 23.4 and 15.0 us (FP32, vehicle), 96x48x48 27.5 and 16.2 us,
-// 256x128x128 73.9 and 71.5 us (FP16, vehicle).
+// 12.3 us, 128x64x64 23.4 and 15.0 us (FP32, vehicle), 96x48x48 27.5 and 16.2 us
+// (FP16, vehicle).
 // The plain cells' form: 64-cell runs of a row as cells x and x + 32 a lane (binary32)
 // or as cell pairs (16-bit storage, nx even), or pairs over a plane (16-bit, nx odd).
 enum Plain { RUNS, PAIRS, LINEAR, LINEAR_NY_ODD };
