@@ -34,9 +34,9 @@ tracers:  the 128x64x64 vehicle in frames of 8 steps with 3-D streaklines, the
           plate smoke and particles advanced after each frame; device times;
 grid_check: the reference's three-tier grid check (GCI band) run one tier
           after another and with the three tiers side by side on one GPU;
-batched_tunnels: 64 seeded tunnels of uneven size and Re, FP16 TRT, two
-          concurrent persistent launches per step from captured graphs,
-          autotuned shape;
+batched_tunnels: 64 seeded tunnels of uneven size and Re, FP16 TRT, the
+          members' own steps side by side or two persistent launches per
+          step, as the autotuner finds;
           aggregate MLUPS and drag error against each tunnel alone in FP32.
 
 --impl reference runs only that CPU path and prints its own line.
@@ -356,9 +356,9 @@ def accuracy_leg(steps, threads):
 
 def batch_leg(steps, sample_steps=200, count=64, peak=None):
     """64 independent tunnels (sizes, bodies and Re from splitmix64 seed 1), FP16
-    storage, TRT, stepped as one batch: per step one persistent launch over all
-    members' plain cells and one over their seam and edge cells beside it,
-    replayed from captured 50-step graphs, launch shape from the autotuner.  Aggregate MLUPS over `steps` steps, then each member's drag over
+    storage, TRT, stepped as one batch, its form (members' own steps side by side,
+    or two persistent launches a step over all members) from the autotuner.
+    Aggregate MLUPS over `steps` steps, then each member's drag over
     the last `sample_steps` steps against the same tunnel run alone in FP32."""
     import numpy as np
     from pocketwind_gb300 import cases, geometry, solver
@@ -403,7 +403,7 @@ def batch_leg(steps, sample_steps=200, count=64, peak=None):
     mlups = cells * steps / (ms * 1e3)
     out = {"domains": count, "cells": cells, "steps": steps, "storage": "f16", "operator": "trt",
            "ms_per_step": round(ms / steps, 4), "mlups": round(mlups, 1),
-           "launches_per_step": 2, "graph_chunk_steps": 50,
+           "forms_timed": "two persistent launches a step; the members' own launches side by side",
            "tuning": {"blocks": tuning.blocks, "rows_per_item": tuning.rows_per_item,
                       "candidates": tuning.candidates},
            "drag_rel_err_vs_solo_f32": {"median": float(np.median(err)), "p90": float(np.percentile(err, 90)),
@@ -511,7 +511,7 @@ def closure_leg(fine_steps, train_steps, threads, snapshots=8):
     out["coarse_re640"] = coarse
     # device time of a closure step over a plain Smagorinsky step on the same grid
     out["closure_kernel"] = ("closure_pairs: the plain step's two-cell update with the network on two 128-cell "
-                             "tcgen05 tiles per block; edge and floor kernels beside it")
+                             "tcgen05 tiles per block; edge cells and floor layer in blocks of the same launch")
     out["closure_over_plain_step"] = {
         walls: coarse["closure" + suffix]["ms_per_step"] / coarse["smagorinsky" + suffix]["ms_per_step"]
         for suffix, walls in (("", "halfway"), ("_bouzidi", "bouzidi"))}

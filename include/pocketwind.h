@@ -264,8 +264,8 @@ PW_API int pw_checkpoint_load(pw_domain *dom, const void *in, size_t size);
    Members step by their own launches side by side on their streams, or, with
    few cells each or a step that is not one launch, by two persistent launches
    a step, one over all members' plain cells and one over their seam and edge
-   cells running beside it, replayed from captured CUDA graphs; members keep their own force, macro and readout
-   calls, which wait for the batch's queued steps.  A member must not be
+   cells running beside it, replayed from captured CUDA graphs; members keep
+   their own force, macro and readout calls, which wait for the batch's queued steps.  A member must not be
    stepped on its own while it belongs to a batch. */
 typedef struct pw_batch pw_batch;
 typedef struct {

@@ -7,8 +7,9 @@
 //   plane[2]  float4 per (y, z): outlet upstream velocity, double-buffered by step parity
 //   flags     u32 per cell; special: 1 bit per cell (non-plain cells)
 //   partials[2] 3 doubles per step block: momentum exchange of the even / odd states
-// Stepping queues one fused kernel per step on the domain's stream; runs of
-// steps without ramping are replayed from captured CUDA graphs.
+// Stepping queues one kernel per step on the domain's stream (large 16-bit domains:
+// the split step's three or four, on two streams); runs of the steps that are not one
+// launch, without ramping, are replayed from captured CUDA graphs on small domains.
 #include <cuda_runtime.h>
 
 #include <algorithm>
