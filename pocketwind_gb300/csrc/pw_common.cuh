@@ -212,12 +212,10 @@ struct StepParams {
   uint32_t *status;        // bit 0: density guard tripped on a macro step
   uint32_t nx, ny, nz;
   uint32_t stride;         // elements between direction planes
-  uint32_t inv_nx;         // floor((2^32 - 1) / nx) + 1: rows of a plane's cells without a division
   float u_in;              // inlet speed of this step
   float nu, cs_term, lambda;
   float tau0, omega_plus, omega_minus;  // binary32 constants of the LES-free operator
   int write_macro;
-  int clear_status;        // this step clears the guard's flag (one-launch steps; a macro step follows)
   uint32_t slip;           // free-slip faces: bit 0 the y faces, bit 1 the z faces (0: periodic)
   // Plain cells (no periodic wrap in reach): direction i is loaded from element
   // n + ld[i] and stored to element n + st[i] of f, offsets for this step's parity.
@@ -245,6 +243,10 @@ struct StepParams {
   const uint32_t *qoff;
   const float *q;
   void *hist;
+  // (behind the offset tables: before them, these two words moved the tables off the
+  // alignment at which the cell-pair kernel reads them, 511 and 516 us a step at 512x256x256)
+  uint32_t inv_nx;         // floor((2^32 - 1) / nx) + 1: rows of a plane's cells without a division
+  int clear_status;        // this step clears the guard's flag (one-launch steps; a macro step follows)
 };
 
 }  // namespace pw
