@@ -668,9 +668,10 @@ __global__ void bin_triangles_kernel(DevBins B, uint32_t ntri, uint32_t *count, 
       }
 }
 
-// intersection, triangle-bins.ts:60-94: the hit depth t along d, or false.  u and v
-// clearly outside [-EPS, 1 + EPS] (by EPS, far beyond the quotient's rounding) are
-// refused before the division: binary64 divisions are most of a test's time.
+// intersection, triangle-bins.ts:60-94: the hit depth t along d, or false.  A u or v that
+// the test must refuse, by more than EPS (far beyond the rounding), is refused before the
+// division: binary64 divisions are most of a test's time.  u lies in [-EPS, 1 + EPS], but v
+// may reach 1 + 2 EPS, beside u = -EPS.
 __device__ __forceinline__ bool segment_hit(const float *p, const double *o, const double *d, double *t) {
   const double EPS = 1e-9;
   double ax = p[0], ay = p[1], az = p[2];
@@ -683,7 +684,7 @@ __device__ __forceinline__ bool segment_hit(const float *p, const double *o, con
   if (fabs(det) < 2.220446049250313e-16) return false;
   const auto outside = [&](double num) {
     const double n = det < 0 ? -num : num, a = fabs(det);
-    return n < -2 * EPS * a || n > (1 + 2 * EPS) * a;
+    return n < -2 * EPS * a || n > (1 + 3 * EPS) * a;
   };
   double tx = o[0] - ax, ty = o[1] - ay, tz = o[2] - az;
   double un = tx * px + ty * py + tz * pz;

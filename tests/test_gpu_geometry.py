@@ -115,3 +115,24 @@ def test_link_fraction_groups(name, make, layout, floor):
     g, r = _both(body, supports, layout, floor, True)
     assert np.array_equal(g.geometry, r.geometry)
     assert g.missed_links == r.missed_links
+
+
+# a triangle before the body's wall that the link from cell (5, 0, 0) meets just outside its
+# third corner, where the reference's test still takes it: u = -1e-9 (a hair above -EPS) and
+# v = 1 + 2e-9, whose sum is 1 + EPS
+@pytest.mark.parametrize("corners", [
+    ("-0x1.423ffap+0", "-0x1.22637ep+0", "0x1.00b2c6p+0", "0x1.cab6a2p+0", "-0x1.198ab4p-32", "0x1.69798ap-31"),
+    ("-0x1.bcebdcp+0", "-0x1.6ac0b6p+0", "0x1.074d3ep+0", "0x1.d44fd8p+0", "-0x1.86066ep-31", "0x1.c55f76p-32"),
+    ("-0x1.fd449ep+0", "-0x1.148588p+0", "0x1.546bfep+0", "0x1.7b9e2ap+0", "-0x1.6a982cp-31", "0x1.bacb88p-32"),
+])
+def test_link_fraction_at_a_corner(corners):
+    yz = [float.fromhex(c) for c in corners]
+    tri = np.array([[5.25, yz[0], yz[1]], [5.25, yz[2], yz[3]], [5.25, yz[4], yz[5]]], np.float32)
+    body = box([5.4, -2.3, -2.3], [8.6, 3.3, 3.3])
+    mesh = meshes.Mesh(np.concatenate([body.positions, tri.reshape(-1)]), body.triangle_count + 1)
+    g, r = _both(mesh, None, (14, 9, 10), False, True)
+    n = 14 * 9 * 10
+    first = int(r.geometry[n + 5])
+    assert r.geometry[2 * n:].view(np.float32)[first] == 0.25  # the link that meets the triangle
+    assert np.array_equal(g.geometry, r.geometry)
+    assert g.missed_links == r.missed_links
