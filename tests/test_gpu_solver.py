@@ -688,3 +688,28 @@ def test_odd_rows_with_les_within_reference_rounding_noise(layout, op, precision
     err, ref_err = norm_err(fast.populations(), want), norm_err(ref16.populations(), want)
     assert np.isfinite(err) and err <= 2 * ref_err, (err, ref_err)
     fast.destroy()
+
+
+def test_domain_leaves_the_stream_ordered_pool_alone():
+    """Memory of the stream-ordered pool that was ever used on a domain's stream slows that
+    stream's event records and waits, so creating, stepping and sampling a domain takes none:
+    the pool's high-water mark (CU_MEMPOOL_ATTR_USED_MEM_HIGH, 8) stays at zero."""
+    import ctypes as C
+    from pocketwind_gb300 import cases
+    G, S = _pw()
+    case = cases.vehicle_case(64)
+    grid = case.grid()
+    cuda = C.CDLL("libcuda.so.1")
+    pool, high = C.c_void_p(), C.c_uint64(0)
+    assert cuda.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+    assert cuda.cuMemPoolSetAttribute(pool, 8, C.byref(high)) == 0  # 0: from now on
+    before = C.c_uint64(0)
+    assert cuda.cuMemPoolGetAttribute(pool, 8, C.byref(before)) == 0
+    for precision in ("f32", "f16"):
+        s = S.GpuSolver.create(case.layout, grid, case.params(precision))
+        s.step(9, True)
+        s.encode_force()
+        s.read_force()
+        s.destroy()
+    assert cuda.cuMemPoolGetAttribute(pool, 8, C.byref(high)) == 0
+    assert high.value == before.value
