@@ -265,12 +265,13 @@ PW_API int pw_checkpoint_load(pw_domain *dom, const void *in, size_t size);
    few cells each or a step that is not one launch, by two persistent launches
    a step, one over all members' plain cells and one over their seam and edge
    cells running beside it, replayed from captured CUDA graphs; members keep
-   their own force, macro and readout calls, which wait for the batch's queued steps.  A member must not be
-   stepped on its own while it belongs to a batch. */
+   their own force, macro and readout calls, which wait for the batch's queued steps.  Both
+   forms store the same values.  A member must not be stepped on its own while it belongs to
+   a batch. */
 typedef struct pw_batch pw_batch;
 typedef struct {
-  uint32_t blocks;         /* persistent grid chosen */
-  uint32_t rows_per_item;  /* plain rows per work item chosen */
+  uint32_t blocks;         /* persistent grid chosen: the fastest, also where the members' */
+  uint32_t rows_per_item;  /* own launches are kept; plain rows per work item chosen */
   float ms_per_step;       /* measured time per step of what is kept: that shape, or
                               the members' own launches where those are faster */
   uint32_t candidates;     /* launch shapes timed */
@@ -282,6 +283,8 @@ PW_API int pw_batch_time_steps(pw_batch *batch, uint64_t count, float *ms);
 /* Autotuner: times each candidate shape over trial_steps real steps (they
    advance the members) and keeps the fastest. */
 PW_API int pw_batch_tune(pw_batch *batch, uint32_t trial_steps, pw_batch_tuning *out);
+/* *own: 1 while the members step by their own launches, 0 while by the persistent ones. */
+PW_API int pw_batch_own_launches(const pw_batch *batch, int *own);
 /* pw_reset of every member; the batch starts again at step 0. */
 PW_API int pw_batch_reset(pw_batch *batch);
 

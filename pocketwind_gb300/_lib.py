@@ -91,6 +91,7 @@ SIGNATURES = {
     "pw_batch_step": (_int, [_vp, _u64, _int]),
     "pw_batch_time_steps": (_int, [_vp, _u64, C.POINTER(C.c_float)]),
     "pw_batch_tune": (_int, [_vp, C.c_uint32, C.c_void_p]),
+    "pw_batch_own_launches": (_int, [_vp, C.POINTER(_int)]),
     "pw_batch_reset": (_int, [_vp]),
     "pw_closure_create": (_int, [_u64, C.POINTER(_vp)]),
     "pw_closure_destroy": (None, [_vp]),

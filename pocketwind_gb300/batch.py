@@ -8,7 +8,9 @@ one launch take their own steps side by side on their streams.  Members of few
 cells, or whose step is several launches, share two persistent launches a step,
 side by side on two streams: one over every member's plain cells, one over their
 seam rows and edge cells, replayed from captured CUDA graphs; ``tune`` times the
-candidate launch shapes and the members' own launches and keeps the fastest.  The members keep their own force, macro and readout calls.
+candidate launch shapes and the members' own launches and keeps the fastest.  Both
+forms store the same values, and the members keep their own force, macro and readout
+calls.
 """
 from __future__ import annotations
 
@@ -61,6 +63,13 @@ class Batch:
         _lib.check(_lib.load().pw_batch_tune(self._live(), int(trial_steps), C.cast(C.pointer(t), C.c_void_p)),
                    "Batch.tune")
         return Tuning(t.blocks, t.rows_per_item, t.ms_per_step, t.candidates)
+
+    @property
+    def own_launches(self) -> bool:
+        """Whether the members step by their own launches (else by the persistent ones)."""
+        v = C.c_int()
+        _lib.check(_lib.load().pw_batch_own_launches(self._live(), C.byref(v)), "Batch.own_launches")
+        return bool(v.value)
 
     def reset(self) -> None:
         _lib.check(_lib.load().pw_batch_reset(self._live()), "Batch.reset")

@@ -51,6 +51,14 @@ constexpr int kChunk = 50;                        // steps per captured graph
 // items in the plain kernel instead, under its register cap, no faster).
 constexpr uint32_t kSeamRowsPerItem = 16;
 
+// An edge item, a function of its own as in a member's own launch (pw_step_all.cuh's
+// edge_role): inlined, the compiler fused other products of the LES wall model than there,
+// and a member's stored values depended on the form that stepped it.
+template <int ST, int OP, bool LES, bool ODD>
+__device__ __noinline__ void edge_item(const StepParams &p, const uint32_t *list, uint32_t count, uint32_t b) {
+  pwbatch::edge_block<ST, OP, LES, ODD>(p, list, count, b, threadIdx.x);
+}
+
 // PLAIN: the plain items (PAIRS: through the 32-bit cell-pair kernel, which
 // needs 16-bit storage and every member's nx even); otherwise
 // the seam and edge items.
@@ -115,7 +123,7 @@ __global__ void __launch_bounds__(kBatchThreads, PLAIN ? PW_BATCH_PLAIN_BLOCKS :
         }
       }
     } else {
-      pwbatch::edge_block<ST, OP, LES, ODD>(sp, lists[m], counts[m], local, tid);
+      edge_item<ST, OP, LES, ODD>(sp, lists[m], counts[m], local);
     }
   }
 }
@@ -179,7 +187,7 @@ struct pw_batch {
   bool pairs = false;             // every member's nx is even: the plain items use the cell-pair kernel
   const uint32_t **lists = nullptr;
   uint32_t *counts = nullptr;
-  bool can_own = false;    // every member's step is one launch
+  bool can_own = false;    // the members may step by their own launches
   bool own = false;        // the members step by their own launches, side by side
   uint32_t rows = 16;      // plain rows per work item
   unsigned blocks = 0;     // persistent grid
@@ -417,13 +425,19 @@ int pw_batch_create(pw_domain *const *members, uint32_t count, pw_batch **out) {
   for (uint32_t m = 0; m < count; m++) b->pairs = b->pairs && (member_view(members[m]).nx & 1u) == 0u;
   b->storage = first.storage; b->op = first.op; b->les = first.les;
   b->steps = first.steps;
+  // Both forms store the same values, so neither the members' sizes nor a timing shows in
+  // them: 16-bit members of even and odd nx together share the persistent launches, whose
+  // x / x + 32 pairs draw other dithers than an even member's own cell pairs.
   b->can_own = true;
+  bool odd = false, even = false;
   uint64_t cells = 0;
   for (uint32_t m = 0; m < count; m++) {
     const MemberView v = member_view(members[m]);
     b->can_own = b->can_own && v.one_launch;
+    ((v.nx & 1u) ? odd : even) = true;
     cells += (uint64_t)v.nx * v.ny * v.nz;
   }
+  if (b->storage != pw::STORE_F32 && odd && even) b->can_own = false;
   // below 48 K cells a member a launch outweighs its step (64x32x32, 65 K cells: even)
   b->own = b->can_own && cells >= (uint64_t)count * (48u << 10);
   b->sms = (unsigned)max_blocks();
@@ -582,6 +596,12 @@ int pw_batch_tune(pw_batch *b, uint32_t trial_steps, pw_batch_tuning *out) {
     out->ms_per_step = best / (float)trial_steps;
     out->candidates = tried;
   }
+  return PW_OK;
+}
+
+int pw_batch_own_launches(const pw_batch *b, int *own) {
+  if (!b || !own) { set_error("NULL argument"); return PW_ERR_INVALID; }
+  *own = b->own ? 1 : 0;
   return PW_OK;
 }
 

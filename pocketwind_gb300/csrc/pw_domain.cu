@@ -988,11 +988,15 @@ MemberView member_view(const pw_domain *d) {
 }
 pw::StepParams member_params(const pw_domain *d, uint64_t step, int write_macro) {
   pw::StepParams p = params_for(d, step, d->u_in, write_macro);
-  p.floor_rows = 0;  // a batch's edge items take the floor layer through the general path
+  p.floor_rows = 0;  // a batch's members take the floor layer through the general path, as edge cells
   return p;
 }
 void member_enqueue(pw_domain *d, uint64_t step, int write_macro, bool before_macro, bool cleared) {
-  enqueue_step(d, step, d->u_in, write_macro, before_macro, cleared, false);
+  pw::StepParams p = member_params(d, step, write_macro);
+  p.clear_status = before_macro ? 1 : 0;
+  if (write_macro && !cleared) cudaMemsetAsync(d->status_dev, 0, 4, d->stream);
+  pwall::launch_step_all(p, d->desc.storage, d->desc.op, d->desc.les, (step & 1) != 0, d->edges, d->edge_count,
+                         d->stream, false);
 }
 void member_advance(pw_domain *d, uint64_t n) { d->steps += n; }
 }  // namespace pwhost

@@ -250,3 +250,59 @@ def test_batch_forms_match_the_reference(layouts, precision, counts):
         assert _norm_err(m.populations(), want) <= (1e-5 if precision == "f32" else 2 * _norm_err(o.populations(), want))
         assert not m.guard_unstable()
     batch.destroy()
+
+
+# no LES and LES, both operators, a floor (its wall model), reflecting faces; nx even and odd
+FORMS = {"trt": {}, "reg": {"operator": "reg"}, "slip": {"lateral": "free-slip"}, "trt les": {"les": True},
+         "reg les": {"operator": "reg", "les": True}, "trt floor": {"les": True, "floor": True},
+         "reg floor": {"operator": "reg", "les": True, "floor": True},
+         "reg les slip": {"operator": "reg", "les": True, "lateral": "free-slip"}}
+
+
+def _form_member(layout, precision, floor=False, **params):
+    from pocketwind_gb300 import geometry, meshes, solver
+    body = meshes.icosphere([layout[0] / 4 + 0.3, layout[1] / 2 + 0.2, layout[2] / 2 - 0.1], min(layout) / 6, 3)
+    return solver.GpuSolver.create(layout, geometry.voxelize(body, None, layout, floor), solver.SolverParams(
+        tau0=0.56, u_in=0.05, precision=precision, **params))
+
+
+def _stepped_in_batch(layouts, precision, form):
+    """The first member's codes, macros and drag after a batch's 1 + 6 + 50 steps, and the batch's form."""
+    from pocketwind_gb300.batch import Batch
+    members = [_form_member(l, precision, **FORMS[form]) for l in layouts]
+    batch = Batch(members)
+    for n in (1, 6, 50):
+        batch.step(n, True)
+    members[0].encode_force()
+    f = members[0].read_force()
+    out = members[0].populations_raw().view(np.uint8), members[0].macros(), (f.fx, f.fy, f.fz), batch.own_launches
+    batch.destroy()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [(48, 24, 24), (49, 25, 23)])
+@pytest.mark.parametrize("precision", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("form", FORMS)
+def test_batch_forms_store_the_same_values(form, precision, layout):
+    """A small tunnel in a batch of its own (persistent launches) and beside a large one (own
+    launches): its codes, macros and drag are the same bits."""
+    large = (128 + layout[0] % 2, 64, 60)
+    a, b = (_stepped_in_batch(l, precision, form) for l in ([layout], [layout, large]))
+    one_launch = not (precision != "f32" and ("slip" in FORMS[form].get("lateral", "") and layout[0] % 2 == 0)) and not (
+        precision == "f16" and layout[0] % 2 and form in ("trt les", "trt floor"))
+    assert (a[3], b[3]) == (False, one_launch)
+    assert np.array_equal(a[0], b[0])
+    assert np.array_equal(a[1], b[1])
+    assert a[2] == b[2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["f16", "bf16"])
+def test_mixed_widths_keep_one_form(precision):
+    """16-bit members of even and odd nx: the persistent launches, whatever the sizes, and the
+    same codes with a small companion and with a large one."""
+    a, b = (_stepped_in_batch([(48, 24, 24), l], precision, "trt") for l in ((31, 16, 16), (129, 64, 60)))
+    assert (a[3], b[3]) == (False, False)
+    assert np.array_equal(a[0], b[0])
+    assert a[2] == b[2]
