@@ -23,6 +23,7 @@
 // stepped alone.
 #define PW_NS pwbatch
 #define PW_STRICT 0
+#define PW_INTERPOLATED 0  // members have halfway walls
 #include <algorithm>
 #include <map>
 #include <vector>

@@ -754,6 +754,12 @@ struct OwnFromHist {
 };
 
 // ---------------------------------------------------------------- the step
+// 0 where no domain has interpolated walls (batches): with their code in it, unused, a
+// batch's edge kernel had 148 registers instead of 128 and a batch of 64 floors of
+// 64x32x32 (FP16, REG, LES) took 199 us a step instead of 120.
+#ifndef PW_INTERPOLATED
+#define PW_INTERPOLATED 1
+#endif
 // One cell of a step.  ODD: this step reads layout E and writes layout O;
 // otherwise the reverse.  flag is the cell's packed flags (0 for plain fluid).
 template <int ST, int OP, bool LES, bool ODD, class Hook = NoHook>
@@ -793,7 +799,7 @@ __device__ __forceinline__ void general_cell(const StepParams &p, uint32_t x, ui
       }
       g[i] = S::decode(f[src]);
     }
-    if (p.qoff != nullptr && (flag >> 3) != 0u)
+    if (PW_INTERPOLATED && p.qoff != nullptr && (flag >> 3) != 0u)
       interpolated_links(p, b, n, flag, g, OwnFromHist<ST>{reinterpret_cast<const T *>(p.hist)}, fx, fy, fz,
                          force_any);
 #if PW_STRICT
@@ -822,7 +828,7 @@ __device__ __forceinline__ void general_cell(const StepParams &p, uint32_t x, ui
     else dst = (pidx)opp_of(j) * S_ + n;
     f[dst] = code[j];
   }
-  if (p.qoff != nullptr && (flag >> 3) != 0u) {
+  if (PW_INTERPOLATED && p.qoff != nullptr && (flag >> 3) != 0u) {
     // keep this step's f*_i(n) of every wall link for the next step's wall values
     const uint32_t base = __ldg(&p.qoff[n]);
     if (base != NO_Q) {
