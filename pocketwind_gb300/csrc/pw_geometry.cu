@@ -254,22 +254,40 @@ __device__ __forceinline__ void pixel_range(float a, float b, float c, uint32_t 
 // projection, its setup in binary64, took 1.90 ms a launch on 200,000 triangles
 // at 256x128x128, six launches a mesh (voxelize and create: 16.7 ms; in this
 // form 4.40 ms).
+// A group with more pixels than kHeavyPixels a warp is only noted here, with its place
+// among all such groups' pieces, and raster_heavy shares the pieces over the GPU: a few
+// large triangles in a fine mesh (a ground plate under a body) kept one warp busy while
+// the others had long ended.
 constexpr int kRasterThreads = 128;
-template <bool FILL>
-__global__ void __launch_bounds__(kRasterThreads) raster_kernel(const float *mesh, uint32_t ntri, Projs P,
-                                                               uint32_t slices, uint32_t *count,
-                                                               const uint32_t *offset, double *hits,
-                                                               uint32_t *nonfinite) {
-  __shared__ float tri[kRasterThreads / 32][32][9];
-  __shared__ unsigned long long first[kRasterThreads / 32][32];  // pixels before each lane's box
-  __shared__ int2 corner[kRasterThreads / 32][32];
-  __shared__ uint32_t width[kRasterThreads / 32][32];
-  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-  const uint32_t warp = blockIdx.x * (kRasterThreads / 32) + wib;
-  const uint32_t group = warp / slices, slice = warp % slices;
+constexpr uint32_t kHeavyPixels = 2048;
+
+struct HeavyGroup {
+  unsigned long long first;  // its first piece among all
+  uint32_t group, proj;
+};
+// Notes taken so far: the groups above this bit, their pieces below it.  3 ntri / 32
+// groups fit above; 2^35 pieces are 7e13 pixels.
+constexpr int kHeavyBits = 35;
+__host__ __device__ constexpr uint32_t heavy_groups(unsigned long long n) { return (uint32_t)(n >> kHeavyBits); }
+__host__ __device__ constexpr unsigned long long heavy_pieces(unsigned long long n) {
+  return n & ((1ull << kHeavyBits) - 1ull);
+}
+
+// A warp's group of triangles and their pixel boxes in one projection.
+struct RasterGroup {
+  float tri[32][9];
+  unsigned long long first[32];  // pixels before each lane's box
+  int2 corner[32];
+  uint32_t width[32];
+};
+
+// Loads the lane's triangle of the group; false past the mesh's end and where a
+// coordinate is not finite.
+__device__ __forceinline__ bool load_triangle(const float *mesh, uint32_t ntri, uint32_t group, RasterGroup &g, float *q,
+                                              uint32_t *nonfinite) {
+  const uint32_t lane = threadIdx.x & 31u;
   const size_t t = (size_t)group * 32u + lane;
   bool ok = t < ntri;
-  float q[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) q[k] = ok ? mesh[9 * t + k] : 0.0f;
   if (ok) {
@@ -278,68 +296,137 @@ __global__ void __launch_bounds__(kRasterThreads) raster_kernel(const float *mes
     for (int k = 0; k < 9; k++) finite = finite && isfinite(q[k]);
     if (!finite) {
       ok = false;
-      if (!FILL) *nonfinite = 1u;
+      if (nonfinite) *nonfinite = 1u;
     }
   }
 #pragma unroll
-  for (int k = 0; k < 9; k++) tri[wib][lane][k] = q[k];
+  for (int k = 0; k < 9; k++) g.tri[lane][k] = q[k];
+  return ok;
+}
+
+// The pixel boxes of the warp's triangles in projection p; returns their pixels' sum.
+__device__ __forceinline__ unsigned long long box_triangles(const Proj &p, const float *q, bool ok, RasterGroup &g) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const int u = p.u, v = p.v;
+  const float qu[3] = {u == 0 ? q[0] : (u == 1 ? q[1] : q[2]), u == 0 ? q[3] : (u == 1 ? q[4] : q[5]),
+                       u == 0 ? q[6] : (u == 1 ? q[7] : q[8])};
+  const float qv[3] = {v == 0 ? q[0] : (v == 1 ? q[1] : q[2]), v == 0 ? q[3] : (v == 1 ? q[4] : q[5]),
+                       v == 0 ? q[6] : (v == 1 ? q[7] : q[8])};
+  int u0, v0;
+  uint32_t w, h;
+  pixel_range(qu[0], qu[1], qu[2], p.su, &u0, &w);
+  pixel_range(qv[0], qv[1], qv[2], p.sv, &v0, &h);
+  unsigned long long own = ok ? (unsigned long long)w * h : 0ull, inc = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long prev = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += prev;
+  }
+  const unsigned long long total = __shfl_sync(0xffffffffu, inc, 31);
+  __syncwarp();
+  g.first[lane] = inc - own;
+  g.corner[lane] = make_int2(u0, v0);
+  g.width[lane] = w;
+  __syncwarp();
+  return total;
+}
+
+// Pixels from, from + step, ... below `to` of the group's boxes, one a lane.
+template <bool FILL>
+__device__ __forceinline__ void raster_pixels(const Proj &p, const RasterGroup &g, unsigned long long from,
+                                              unsigned long long to, unsigned long long step, uint32_t *count,
+                                              const uint32_t *offset, double *hits) {
+  const int u = p.u, v = p.v;
+  for (unsigned long long k = from; k < to; k += step) {
+    // the last lane whose box begins at or before pixel k
+    uint32_t j = 0;
+#pragma unroll
+    for (uint32_t half = 16; half > 0; half >>= 1)
+      if (g.first[j + half] <= k) j += half;
+    const unsigned long long at = k - g.first[j];
+    const uint32_t bw = g.width[j];
+    const int2 c0 = g.corner[j];
+    const long long pu = c0.x + (long long)(at % bw), pv = c0.y + (long long)(at / bw);
+    const float *m = g.tri[j];
+    const double A[3] = {m[u], m[v], m[p.axis]};
+    const double B0[3] = {m[3 + u], m[3 + v], m[3 + p.axis]};
+    const double C0[3] = {m[6 + u], m[6 + v], m[6 + p.axis]};
+    const double signed_area = edge_fn(A, B0, C0[0], C0[1]);
+    if (signed_area == 0) continue;
+    const bool front = signed_area > 0;
+    const double B[3] = {front ? B0[0] : C0[0], front ? B0[1] : C0[1], front ? B0[2] : C0[2]};
+    const double C[3] = {front ? C0[0] : B0[0], front ? C0[1] : B0[1], front ? C0[2] : B0[2]};
+    const double wa = edge_fn(B, C, (double)pu, (double)pv);
+    if (!owns_edge(wa, B, C)) continue;
+    const double wb = edge_fn(C, A, (double)pu, (double)pv);
+    if (!owns_edge(wb, C, A)) continue;
+    const double wc = edge_fn(A, B, (double)pu, (double)pv);
+    if (!owns_edge(wc, A, B)) continue;
+    const size_t col = p.col0 + (size_t)pu + (size_t)p.su * (size_t)pv;
+    if (!FILL) {
+      atomicAdd(&count[col], 1u);
+    } else {
+      const uint32_t place = atomicSub(&count[col], 1u) - 1u;
+      hits[offset[col] + place] = (wa * A[2] + wb * B[2] + wc * C[2]) / fabs(signed_area);
+    }
+  }
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(kRasterThreads) raster_kernel(const float *mesh, uint32_t ntri, Projs P,
+                                                               uint32_t slices, uint32_t *count,
+                                                               const uint32_t *offset, double *hits,
+                                                               uint32_t *nonfinite, HeavyGroup *heavy,
+                                                               unsigned long long *noted) {
+  __shared__ RasterGroup groups[kRasterThreads / 32];
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warp = blockIdx.x * (kRasterThreads / 32) + (threadIdx.x >> 5);
+  const uint32_t group = warp / slices, slice = warp % slices;
+  RasterGroup &g = groups[threadIdx.x >> 5];
+  float q[9];
+  const bool ok = load_triangle(mesh, ntri, group, g, q, FILL ? nullptr : nonfinite);
   for (int pr = 0; pr < 3; pr++) {
-    const Proj &p = P.p[pr];
-    const int u = p.u, v = p.v;
-    const float qu[3] = {u == 0 ? q[0] : (u == 1 ? q[1] : q[2]), u == 0 ? q[3] : (u == 1 ? q[4] : q[5]),
-                         u == 0 ? q[6] : (u == 1 ? q[7] : q[8])};
-    const float qv[3] = {v == 0 ? q[0] : (v == 1 ? q[1] : q[2]), v == 0 ? q[3] : (v == 1 ? q[4] : q[5]),
-                         v == 0 ? q[6] : (v == 1 ? q[7] : q[8])};
-    int u0, v0;
-    uint32_t w, h;
-    pixel_range(qu[0], qu[1], qu[2], p.su, &u0, &w);
-    pixel_range(qv[0], qv[1], qv[2], p.sv, &v0, &h);
-    unsigned long long own = ok ? (unsigned long long)w * h : 0ull, inc = own;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long prev = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= (uint32_t)o) inc += prev;
-    }
-    const unsigned long long total = __shfl_sync(0xffffffffu, inc, 31);
-    __syncwarp();
-    first[wib][lane] = inc - own;
-    corner[wib][lane] = make_int2(u0, v0);
-    width[wib][lane] = w;
-    __syncwarp();
-    for (unsigned long long k = (unsigned long long)slice * 32u + lane; k < total;
-         k += (unsigned long long)slices * 32u) {
-      // the last lane whose box begins at or before pixel k
-      uint32_t j = 0;
-#pragma unroll
-      for (uint32_t step = 16; step > 0; step >>= 1)
-        if (first[wib][j + step] <= k) j += step;
-      const unsigned long long at = k - first[wib][j];
-      const uint32_t bw = width[wib][j];
-      const int2 c0 = corner[wib][j];
-      const long long pu = c0.x + (long long)(at % bw), pv = c0.y + (long long)(at / bw);
-      const float *m = tri[wib][j];
-      const double A[3] = {m[u], m[v], m[p.axis]};
-      const double B0[3] = {m[3 + u], m[3 + v], m[3 + p.axis]};
-      const double C0[3] = {m[6 + u], m[6 + v], m[6 + p.axis]};
-      const double signed_area = edge_fn(A, B0, C0[0], C0[1]);
-      if (signed_area == 0) continue;
-      const bool front = signed_area > 0;
-      const double B[3] = {front ? B0[0] : C0[0], front ? B0[1] : C0[1], front ? B0[2] : C0[2]};
-      const double C[3] = {front ? C0[0] : B0[0], front ? C0[1] : B0[1], front ? C0[2] : B0[2]};
-      const double wa = edge_fn(B, C, (double)pu, (double)pv);
-      if (!owns_edge(wa, B, C)) continue;
-      const double wb = edge_fn(C, A, (double)pu, (double)pv);
-      if (!owns_edge(wb, C, A)) continue;
-      const double wc = edge_fn(A, B, (double)pu, (double)pv);
-      if (!owns_edge(wc, A, B)) continue;
-      const size_t col = p.col0 + (size_t)pu + (size_t)p.su * (size_t)pv;
-      if (!FILL) {
-        atomicAdd(&count[col], 1u);
-      } else {
-        const uint32_t place = atomicSub(&count[col], 1u) - 1u;
-        hits[offset[col] + place] = (wa * A[2] + wb * B[2] + wc * C[2]) / fabs(signed_area);
+    const unsigned long long total = box_triangles(P.p[pr], q, ok, g);
+    if (total > (unsigned long long)slices * kHeavyPixels) {
+      if (!FILL && slice == 0u && lane == 0u) {
+        const unsigned long long pieces = (total + kHeavyPixels - 1u) / kHeavyPixels;
+        const unsigned long long before = atomicAdd(noted, (1ull << kHeavyBits) + pieces);
+        heavy[heavy_groups(before)] = HeavyGroup{heavy_pieces(before), group, (uint32_t)pr};
       }
+      continue;
     }
+    raster_pixels<FILL>(P.p[pr], g, (unsigned long long)slice * 32u + lane, total, (unsigned long long)slices * 32u,
+                        count, offset, hits);
+  }
+}
+
+// The noted groups' pieces of kHeavyPixels, one a warp at a time (the notes lie in the
+// order of their first pieces).  200,000 triangles and a ground plate of 12 at
+// 512x256x256: 57 ms to voxelize with the plate's groups on a warp each, 1.6 ms so.
+template <bool FILL>
+__global__ void __launch_bounds__(kRasterThreads) raster_heavy(const float *mesh, uint32_t ntri, Projs P,
+                                                              const HeavyGroup *heavy, uint32_t n,
+                                                              unsigned long long pieces, uint32_t *count,
+                                                              const uint32_t *offset, double *hits) {
+  __shared__ RasterGroup groups[kRasterThreads / 32];
+  const uint32_t lane = threadIdx.x & 31u;
+  RasterGroup &g = groups[threadIdx.x >> 5];
+  const uint64_t warps = (uint64_t)gridDim.x * (kRasterThreads / 32);
+  for (uint64_t k = (uint64_t)blockIdx.x * (kRasterThreads / 32) + (threadIdx.x >> 5); k < pieces; k += warps) {
+    uint32_t lo = 0, hi = n;  // the last note whose first piece is at or before piece k
+    while (hi - lo > 1u) {
+      const uint32_t mid = lo + (hi - lo) / 2u;
+      if (heavy[mid].first <= k) lo = mid;
+      else hi = mid;
+    }
+    const HeavyGroup note = heavy[lo];
+    const Proj &p = P.p[note.proj];
+    float q[9];
+    const bool ok = load_triangle(mesh, ntri, note.group, g, q, nullptr);
+    const unsigned long long total = box_triangles(p, q, ok, g);
+    const unsigned long long from = (k - note.first) * kHeavyPixels;
+    raster_pixels<FILL>(p, g, from + lane, min(total, from + kHeavyPixels), 32u, count, offset, hits);
+    __syncwarp();  // the group's words are free again
   }
 }
 
@@ -555,6 +642,7 @@ struct GridInfo {
   uint32_t hits;
   uint32_t links, boundary;          // wall links; fluid cells next to the body
   uint32_t missed;                   // links whose cast met no triangle
+  unsigned long long heavy[2];       // body, supports: the raster's notes (kHeavyBits)
 };
 
 static int read_info(const GridInfo *info, GridInfo *out, cudaStream_t s) {
@@ -579,26 +667,39 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
     P.p[p] = Proj{u, v, a, sizes[u], sizes[v], sizes[a], strides[u], strides[v], strides[a], ncol};
     ncol += (size_t)sizes[u] * sizes[v];
   }
-  uint32_t *count = nullptr, *offset = nullptr;
   GridInfo got{};
   double *hits = nullptr;
-  cudaError_t e = tmp_alloc(votes_out, (cells + 3) / 4 * 4, s);
-  uint8_t *votes = *votes_out;
-  if (e == cudaSuccess) e = tmp_alloc(&count, ncol * 4, s);
-  if (e == cudaSuccess) e = tmp_alloc(&offset, (ncol + 1) * 4, s);
-  int rc = e == cudaSuccess ? PW_OK : cuda_status(e, "voxelize columns");
   // one warp a group of 32 triangles, or as many as fill the GPU's 152 SMs with 16
   const uint32_t groups = (ntri + 31u) / 32u;
+  cudaError_t e = tmp_alloc(votes_out, (cells + 3) / 4 * 4, s);
+  uint8_t *votes = *votes_out;
+  // the notes, the columns' counts and offsets in one allocation
+  const size_t notes = 3 * (size_t)groups * sizeof(HeavyGroup);
+  char *columns = nullptr;
+  if (e == cudaSuccess) e = tmp_alloc(&columns, notes + (2 * ncol + 1) * 4, s);
+  HeavyGroup *heavy = reinterpret_cast<HeavyGroup *>(columns);
+  uint32_t *count = reinterpret_cast<uint32_t *>(columns + notes), *offset = count + ncol;
+  int rc = e == cudaSuccess ? PW_OK : cuda_status(e, "voxelize columns");
   const uint32_t slices = std::max(1u, std::min(1024u, 152u * 16u / groups));
   const unsigned rblocks = (unsigned)(((uint64_t)groups * slices + kRasterThreads / 32 - 1) / (kRasterThreads / 32));
   if (rc == PW_OK) {
     cudaMemsetAsync(votes, 0, (cells + 3) / 4 * 4, s);
     cudaMemsetAsync(count, 0, ncol * 4, s);
     raster_kernel<false><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, nullptr, nullptr,
-                                                            &info->nonfinite);
+                                                            &info->nonfinite, heavy, &info->heavy[which]);
     rc = exclusive_scan(count, offset, ncol, &info->hits, s);
   }
   if (rc == PW_OK) rc = read_info(info, &got, s);
+  const uint32_t noted = heavy_groups(got.heavy[which]);
+  const unsigned long long pieces = heavy_pieces(got.heavy[which]);
+  const unsigned hblocks = (unsigned)std::min<unsigned long long>((pieces + kRasterThreads / 32 - 1) / (kRasterThreads / 32),
+                                                                  152u * 16u);
+  if (rc == PW_OK && noted && !got.nonfinite) {  // their hits too, and the columns' offsets anew
+    raster_heavy<false><<<hblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, heavy, noted, pieces, count, nullptr,
+                                                           nullptr);
+    rc = exclusive_scan(count, offset, ncol, &info->hits, s);
+    if (rc == PW_OK) rc = read_info(info, &got, s);
+  }
   if (rc == PW_OK && got.nonfinite) {
     set_error("Mesh coordinates must be finite.");
     rc = PW_ERR_INVALID;
@@ -607,14 +708,18 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
     e = tmp_alloc(&hits, (size_t)got.hits * sizeof(double), s);
     if (e != cudaSuccess) rc = cuda_status(e, "voxelize hits");
     if (rc == PW_OK) {
-      raster_kernel<true><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, offset, hits, nullptr);
+      raster_kernel<true><<<rblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, slices, count, offset, hits, nullptr,
+                                                             nullptr, nullptr);
+      if (noted)
+        raster_heavy<true><<<hblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, heavy, noted, pieces, count, offset,
+                                                              hits);
       size_t most = 0;
       for (int p = 0; p < 3; p++) most = std::max(most, (size_t)P.p[p].su * P.p[p].sv);
       column_kernel<<<dim3(nblk(most, 128), 3), 128, 0, s>>>(P, offset, hits, reinterpret_cast<uint32_t *>(votes),
                                                              &info->odd[which]);
     }
   }
-  tmp_free(count, s); tmp_free(offset, s); tmp_free(hits, s);
+  tmp_free(columns, s); tmp_free(hits, s);
   return rc;
 }
 
