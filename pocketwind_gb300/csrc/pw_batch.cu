@@ -190,7 +190,7 @@ struct pw_batch {
   uint32_t *counts = nullptr;
   bool can_own = false;    // the members may step by their own launches
   bool own = false;        // the members step by their own launches, side by side
-  uint32_t rows = 16;      // plain rows per work item
+  uint32_t rows = 8;       // plain rows per work item (16: 3 FP32 tunnels of 64x32x32 15.4 us a step, not 10.8)
   unsigned blocks = 0;     // persistent grid
   uint64_t steps = 0;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
@@ -349,8 +349,8 @@ void batch_to_members(pw_batch *b) {
 // another, and a step runs at a single domain's rate (its offsets are kernel constants,
 // no block barriers between items).  A step of 32 mixed tunnels (FP16; FP32): 433 and 622
 // us, as the tuned persistent launches 493 and 736; of eight 101x53x47: 40 and 62 against
-// 68 and 78; of 64 tunnels of 64x32x32: 98 and 148 against 99 and 152.  Four or 16 steps
-// of a member at a time: the mixed tunnels 2% slower, 24 of 96x48x48 3 to 7% faster.
+// 68 and 78.  The host queues a launch a member and step, 2.4 us each.  Four or 16 steps of
+// a member at a time: the mixed tunnels 2% slower, 24 of 96x48x48 3 to 7% faster.
 void queue_own(pw_batch *b, uint64_t count, int macro_last) {
   for (uint64_t k = 0; k < count; k++)
     for (pw_domain *d : b->members)
@@ -439,10 +439,13 @@ int pw_batch_create(pw_domain *const *members, uint32_t count, pw_batch **out) {
     cells += (uint64_t)v.nx * v.ny * v.nz;
   }
   if (b->storage != pw::STORE_F32 && odd && even) b->can_own = false;
-  // below 48 K cells a member a launch outweighs its step (64x32x32, 65 K cells: even)
-  b->own = b->can_own && cells >= (uint64_t)count * (48u << 10);
+  // Below 80 K cells a member its launch takes the host as long as its step the GPU: 64
+  // tunnels of 64x32x32 (65 K cells) FP16 157 us a step by their own launches, 151 of them
+  // the host's, and 99 by the persistent ones from a graph; 32 of 72x36x36 (93 K) 90 and 114.
+  b->can_own = b->can_own && cells >= (uint64_t)count * (80u << 10);
+  b->own = b->can_own;
   b->sms = (unsigned)max_blocks();
-  b->blocks = b->sms * 32u;  // with 16 rows an item what tuning mostly finds (4 and 4: half the rate)
+  b->blocks = b->sms * 32u;  // with 8 rows an item within 4% of what tuning finds (4 and 4: half the rate)
   auto fail = [&](int rc) {
     pw_batch_destroy(b);
     return rc;

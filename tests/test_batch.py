@@ -306,3 +306,17 @@ def test_mixed_widths_keep_one_form(precision):
     assert (a[3], b[3]) == (False, False)
     assert np.array_equal(a[0], b[0])
     assert a[2] == b[2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout,own", [((64, 32, 32), False), ((80, 32, 31), False), ((80, 32, 32), True),
+                                        ((72, 36, 36), True)])
+def test_members_of_few_cells_share_the_persistent_launches(layout, own):
+    """The line is 80 K cells a member; below it tuning keeps the persistent launches too."""
+    from pocketwind_gb300.batch import Batch
+    members = [_form_member(layout, "f16") for _ in range(2)]
+    batch = Batch(members)
+    assert batch.own_launches == own
+    batch.tune(2)
+    assert own or not batch.own_launches
+    batch.destroy()
