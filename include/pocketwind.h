@@ -236,6 +236,10 @@ PW_API int pw_inject_nan(pw_domain *dom);
 /* Device buffers for interop (macros: float4 per cell; flags: u32 per cell)
  * and the domain's CUDA stream. */
 PW_API int pw_domain_buffers(pw_domain *dom, void **macros, void **flags, void **stream);
+/* shared 1: the domain is stepped while other domains' steps run on the GPU (0, the default:
+ * it has the GPU to itself).  Its steps are launched so that they leave the others room; the
+ * values are the same. */
+PW_API int pw_domain_share(pw_domain *dom, int shared);
 /* fieldVtkBytes (src/io/field-export.ts:31-33 over writeVtk, src/io/vtk.ts:27-81)
  * for the macros as last written, formatted on the GPU: the 16 * cells + 25
  * bytes that follow writeVtk's header (rho as big-endian binary32, a newline,

@@ -80,6 +80,7 @@ SIGNATURES = {
     "pw_guard_check": (_int, [_vp, C.POINTER(C.c_int)]),
     "pw_inject_nan": (_int, [_vp]),
     "pw_domain_buffers": (_int, [_vp, _PP, _PP, _PP]),
+    "pw_domain_share": (_int, [_vp, _int]),
     "pw_field_vtk_body": (_int, [_vp, C.c_double, _vp, _sz]),
     "pw_checkpoint_size": (_int, [_vp, C.POINTER(_sz)]),
     "pw_checkpoint_save": (_int, [_vp, _vp, _sz]),

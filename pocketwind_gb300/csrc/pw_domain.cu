@@ -209,6 +209,7 @@ struct pw_domain {
   uint32_t slip = 0;              // free-slip faces (bit 0 y, bit 1 z)
   bool split = false;             // fast build, one cell per thread: plain kernel + edge list
   bool one_launch = false;        // a split step as one launch
+  bool shared = false;            // stepped beside other domains (pw_domain_share)
   uint32_t *edges = nullptr;      // edge cells in ascending order
   uint32_t edge_count = 0;
   uint32_t edge_own = 0;          // the list's head that a domain's own step runs (all but its floor cells)
@@ -287,8 +288,17 @@ pw::StepParams params_for(const pw_domain *d, uint64_t step, float u_in, int wri
   return p;
 }
 
+// Domains stepped beside others take the one-launch step up to a million cells: above, the
+// split step, whose side kernels' streams have priority over the other domains' plain cells.
+// 8 steps each of 128x64x64, 192x96x96 and 256x128x128 with drags (REG LES, floor), a step:
+// FP32 171.2 us as one launch each, 166.6 so; FP16 117.4 and 117.3, BF16 116.4 and 114.8;
+// early, as when one after another, 173.7, 125.7 and 124.1 (blocks that wait for their
+// step hold the places of the other domains').
+constexpr size_t kSharedOneLaunch = (size_t)1 << 20;
+bool split_in_one(const pw_domain *d) { return d->one_launch && !(d->shared && d->cells > kSharedOneLaunch); }
+
 // Whether a step is one launch (the split step in that form, the closure's cell pairs).
-bool single_launch(const pw_domain *d) { return d->split && (d->one_launch || d->closure_frag); }
+bool single_launch(const pw_domain *d) { return d->split && (split_in_one(d) || d->closure_frag); }
 
 // Queue step number `step` (1-based) with the given inlet speed.  The guard's flag of a
 // macro step starts at zero: a step of one launch before it in the same call clears it
@@ -314,7 +324,7 @@ void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool
   else if (d->closure_frag)
     pwclosure_host::launch_closure_step(p, d->desc.storage, d->desc.op, odd, d->grid, d->closure_frag, d->wall_dist,
                                         d->stream);
-  else if (d->one_launch && d->split)
+  else if (d->split && split_in_one(d))
     pwall::launch_step_all(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->edges, d->edge_own, d->stream,
                            early);
   else if (d->split)
@@ -728,11 +738,12 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
     return PW_ERR_INVALID;
   }
   uint64_t k = 0;
+  const bool early = !d->shared;
   // ramped steps, one launch each with its own inlet speed
   while (k < count && d->desc.ramp_steps > 0 && d->steps < d->desc.ramp_steps) {
     uint64_t step = d->steps + 1;
     enqueue_step(d, step, ramp_speed(d, step), write_macro_on_last && k == count - 1,
-                 write_macro_on_last && k + 2 == count, k > 0);
+                 write_macro_on_last && k + 2 == count, k > 0, early);
     d->steps++;
     k++;
   }
@@ -752,7 +763,8 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
   }
   for (; k < count; k++) {
     uint64_t step = d->steps + 1;
-    enqueue_step(d, step, d->u_in, write_macro_on_last && k == count - 1, write_macro_on_last && k + 2 == count, k > 0);
+    enqueue_step(d, step, d->u_in, write_macro_on_last && k == count - 1, write_macro_on_last && k + 2 == count, k > 0,
+                 early);
     d->steps++;
   }
   PW_TRY(cudaGetLastError());
@@ -904,6 +916,12 @@ int pw_domain_buffers(pw_domain *d, void **macros, void **flags, void **stream) 
   if (macros) *macros = d->macros;
   if (flags) *flags = d->flags;
   if (stream) *stream = d->stream;
+  return PW_OK;
+}
+
+int pw_domain_share(pw_domain *d, int shared) {
+  if (!alive(d)) return PW_ERR_INVALID;
+  d->shared = shared != 0;
   return PW_OK;
 }
 

@@ -396,6 +396,7 @@ def gpu_grid_check(body_mesh_for, current_length_cells: float, current_nx: float
             length = grid_check_length_cells(current_length_cells, current_nx, tier)
             total, average = grid_check_steps(tier, run_flow_throughs)
             sv, scale = _tier_solver(tier, length, body_mesh_for, re, precision, floor)
+            sv.share()
             runs.append(dict(tier=tier, length=length, total=total, average=average, solver=sv, scale=scale,
                              history=[]))
         while any(r["solver"].step_count < r["total"] for r in runs):

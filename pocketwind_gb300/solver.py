@@ -134,6 +134,11 @@ class GpuSolver:
             raise RangeError("Step count must be a non-negative safe integer.")
         _lib.check(_lib.load().pw_step(self._live(), int(count), int(bool(write_macro_on_last))), "step")
 
+    def share(self, shared: bool = True) -> None:
+        """Say that the solver is stepped while others' steps run on the GPU: its steps then leave
+        them room (one after another they are faster without).  The values are the same."""
+        _lib.check(_lib.load().pw_domain_share(self._live(), int(bool(shared))), "share")
+
     @property
     def step_count(self) -> int:
         v = C.c_uint64()

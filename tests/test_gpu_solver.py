@@ -713,3 +713,29 @@ def test_domain_leaves_the_stream_ordered_pool_alone():
         s.destroy()
     assert cuda.cuMemPoolGetAttribute(pool, 8, C.byref(high)) == 0
     assert high.value == before.value
+
+
+@pytest.mark.parametrize("precision", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("layout", [(64, 32, 32), (65, 33, 32), (160, 90, 80), (161, 91, 81)])
+def test_shared_domain_stores_the_same_values(layout, precision):
+    """A domain that shares the GPU runs other block forms, above a million cells the split
+    step; the codes, macros, guard and drag are the same bits, also when that changes on the way."""
+    from pocketwind_gb300 import meshes
+    G, S = _pw()
+    body = meshes.icosphere([n / 2.1 for n in layout], min(layout) / 5, 3)
+    grid = G.voxelize(body, None, layout, True)
+    got = []
+    for plan in ((False, False, False), (True, True, True), (True, False, True)):
+        s = S.GpuSolver.create(layout, grid, S.SolverParams(tau0=0.56, u_in=0.05, les=True, operator="reg",
+                                                            precision=precision))
+        for shared, n in zip(plan, (1, 9, 70)):
+            s.share(shared)
+            s.step(n, True)
+        s.encode_force()
+        f = s.read_force()
+        got.append((s.populations_raw().view(np.uint8), s.macros(), (f.fx, f.fy, f.fz), s.guard_unstable()))
+        s.destroy()
+    for other in got[1:]:
+        assert np.array_equal(got[0][0], other[0])
+        assert np.array_equal(got[0][1], other[1])
+        assert got[0][2:] == other[2:]

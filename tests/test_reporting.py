@@ -267,6 +267,40 @@ def test_concurrent_grid_check_equals_one_at_a_time():
         assert r.cd is not None and 0.1 < r.cd < 10
 
 
+@pytest.mark.gpu
+def test_tiers_side_by_side_leave_each_other_room():
+    """The grid check says of its domains that they share the GPU, and the three tiers so are
+    stepped faster than as domains that each have it to themselves (117 and 126 us a step)."""
+    import time
+    from pocketwind_gb300 import solver
+    said = []
+    share = solver.GpuSolver.share
+    try:
+        solver.GpuSolver.share = lambda self, shared=True: (said.append(self.layout), share(self, shared))[1]
+        R.gpu_grid_check(_sphere_for, 16, 128, re=200.0, run_flow_throughs=0.01, floor=False)
+    finally:
+        solver.GpuSolver.share = share
+    assert said == [R.TIERS[t] for t in R.GRID_CHECK_TIERS]
+    tiers = [R._tier_solver(t, R.grid_check_length_cells(16, 128, t), _sphere_for, 200.0, "f16", True)[0]
+             for t in R.GRID_CHECK_TIERS]
+    best = []
+    for shared in (False, True):
+        for sv in tiers:
+            sv.share(shared)
+        times = []
+        for _ in range(20):
+            t = time.perf_counter()
+            for _ in range(4):
+                for sv in tiers:
+                    sv.step(8)
+                    sv.encode_force()
+                for sv in tiers:
+                    sv.read_force()
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+    assert best[1] < 0.98 * best[0], best
+
+
 # ---------------------------------------------------------------- units.test.ts
 def test_units_constants():
     """tests/unit/units/units.test.ts:11-15."""
