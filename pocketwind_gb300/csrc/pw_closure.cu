@@ -599,7 +599,8 @@ __device__ __noinline__ void floor_role(const StepParams &p, uint32_t b, uint32_
 // A step whose blocks all find a place at four per SM runs in the form with their 128
 // registers: its time is one tile's and one wall-link cell's, whose spilled registers
 // count then (64x32x32 FP32 15.3 and 13.4 us with 64 and 128 registers, FP16 18.2 and
-// 14.9; separate kernels 15.9 and 23.8 in short calls, 12.3 and 18.9 in captured ones).
+// 14.9; separate kernels 15.9 and 23.8 in short calls).  Long runs of few tiles are captured
+// with separate kernels (closure_long_runs_captured).
 #ifndef PW_CLOSURE_PAIR_BLOCKS
 #define PW_CLOSURE_PAIR_BLOCKS 8
 #endif
@@ -1293,8 +1294,24 @@ static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const 
 
 template <int ST, int OP, bool ODD>
 static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const uint8_t *wall, const uint32_t *list,
-                               uint32_t count, uint32_t *taken, bool early, cudaStream_t s) {
+                               uint32_t count, uint32_t *taken, bool early, cudaStream_t s,
+                               const pwfast::SideStream *beside) {
   const uint32_t runs = (p.nx + 63u) / 64u, row_blocks = (p.ny + 3u) / 4u;
+  if (beside) {
+    if constexpr (ST != pw::STORE_F32) {
+      if (p.floor_rows && p.ny >= 3u)
+        pwclosure::aa_step_floor<ST, OP, true, ODD>
+            <<<dim3(runs, (p.ny - 2u + pwclosure::BY - 1u) / pwclosure::BY), dim3(pwclosure::BX, pwclosure::BY), 0,
+               beside->stream>>>(p);
+    }
+    if (count)
+      pwclosure::aa_step_edges<ST, OP, true, ODD>
+          <<<(count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, pwclosure::NTHREADS, 0, beside->stream>>>(p, list,
+                                                                                                             count);
+    const ClosureSide none{list, 0u, 0u, 0u, taken};
+    closure_pairs_step<ST, OP, ODD, PW_CLOSURE_PAIR_BLOCKS>(p, frag, wall, runs, row_blocks, none, false, s);
+    return;
+  }
   ClosureSide side{list, count, (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, 0u, taken};
   if (ST != pw::STORE_F32 && p.floor_rows && p.ny >= 3u) side.floor = runs * ((p.ny - 2u + 3u) / 4u);
   if ((uint64_t)runs * row_blocks * p.nz + side.edge + side.floor <= (uint64_t)PW_CLOSURE_FEW_BLOCKS * sm_count())
@@ -1303,13 +1320,33 @@ static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const 
     closure_pairs_step<ST, OP, ODD, PW_CLOSURE_PAIR_BLOCKS>(p, frag, wall, runs, row_blocks, side, early, s);
 }
 
+// The line between a long run's two forms.  A step of few tiles is as long as one tile or one
+// edge cell, and captured steps follow one another closer than early launches; more tiles
+// fill the GPU, and blocks that take tiles as they come win.  A step in a run of 256, early
+// launches and captured: FP32 REG with a floor 64x32x32 13.7 and 12.4 us, 33x17x17 13.1 and
+// 10.9, 66x33x33 15.7 and 15.1, 72x36x36 (648 tiles) 15.4 and 16.4; FP16 with nx odd and a
+// floor 33x17x17 15.0 and 11.7, 65x33x33 18.1 and 15.9, 73x37x37 16.9 and 17.5.  With few
+// edge cells the line is later (a sphere without a floor, FP16: 72x36x36 18.5 and 15.8,
+// 73x37x37 18.7 and 16.8, 88x44x44 18.0 and 19.7).  With the floor layer in a kernel of its
+// own the early launches are the faster ones at any size (FP16 64x32x32 16.1 and 16.3).
+bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int floor_rows, uint32_t count) {
+  if (floor_rows && ny >= 3u) return false;
+  const uint64_t tiles = (uint64_t)((nx + 63u) / 64u) * ((ny + 3u) / 4u) * nz, sms = (uint64_t)sm_count();
+  const uint64_t edge = (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS;
+  return 5u * tiles <= (8u * edge < sms ? 25u : 21u) * sms;
+}
+
 void launch_closure_pairs(const StepParams &p, int storage, int op, bool odd, const uint32_t *frag,
                           const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken,
-                          bool early, cudaStream_t s) {
-#define PW_CLP(ST, OPV)                                                          \
-  do {                                                                           \
-    if (odd) closure_pairs_step<ST, OPV, true>(p, frag, wall, list, count, taken, early, s);   \
-    else closure_pairs_step<ST, OPV, false>(p, frag, wall, list, count, taken, early, s);      \
+                          bool early, cudaStream_t s, const pwfast::SideStream *side) {
+  if (side) {
+    cudaEventRecord(side->fork, s);
+    cudaStreamWaitEvent(side->stream, side->fork, 0);
+  }
+#define PW_CLP(ST, OPV)                                                                            \
+  do {                                                                                             \
+    if (odd) closure_pairs_step<ST, OPV, true>(p, frag, wall, list, count, taken, early, s, side); \
+    else closure_pairs_step<ST, OPV, false>(p, frag, wall, list, count, taken, early, s, side);    \
   } while (0)
   if (op == pw::OP_REG) {
     if (storage == pw::STORE_F16) PW_CLP(pw::STORE_F16, pw::OP_REG);
@@ -1321,6 +1358,10 @@ void launch_closure_pairs(const StepParams &p, int storage, int op, bool odd, co
     else PW_CLP(pw::STORE_F32, pw::OP_TRT);
   }
 #undef PW_CLP
+  if (side) {
+    cudaEventRecord(side->join, side->stream);
+    cudaStreamWaitEvent(s, side->join, 0);
+  }
 }
 
 int wall_distance_of(const uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *out, cudaStream_t s) {

@@ -303,10 +303,11 @@ bool single_launch(const pw_domain *d) { return d->split && (split_in_one(d) || 
 // Queue step number `step` (1-based) with the given inlet speed.  The guard's flag of a
 // macro step starts at zero: a step of one launch before it in the same call clears it
 // (before_macro, then cleared), without a memset between the two.
+enum StepLaunch { STEP_EARLY, STEP_BESIDE, STEP_CAPTURED };  // while the step before it ends, or not, or in a graph
 void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool before_macro = false,
-                  bool cleared = false, bool early = true) {
+                  bool cleared = false, StepLaunch how = STEP_EARLY) {
   pw::StepParams p = params_for(d, step, u_in, write_macro);
-  const bool one = single_launch(d);
+  const bool one = single_launch(d), early = how == STEP_EARLY;
   p.clear_status = one && before_macro ? 1 : 0;
   if (write_macro && !(one && cleared)) cudaMemsetAsync(d->status_dev, 0, 4, d->stream);
   bool odd = (step & 1) != 0;
@@ -320,7 +321,8 @@ void enqueue_step(pw_domain *d, uint64_t step, float u_in, int write_macro, bool
     pwstrict::launch_step(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->grid, d->stream);
   else if (d->closure_frag && d->split)
     pwclosure_host::launch_closure_pairs(p, d->desc.storage, d->desc.op, odd, d->closure_frag, d->wall_dist, d->edges,
-                                         d->edge_own, d->tiles_taken, early, d->stream);
+                                         d->edge_own, d->tiles_taken, early, d->stream,
+                                         how == STEP_CAPTURED ? &d->side : nullptr);
   else if (d->closure_frag)
     pwclosure_host::launch_closure_step(p, d->desc.storage, d->desc.op, odd, d->grid, d->closure_frag, d->wall_dist,
                                         d->stream);
@@ -449,7 +451,7 @@ cudaGraphExec_t graph_for(pw_domain *d, int start_parity, int macro_last) {
     for (int k = 0; k < kGraphChunk; k++) {
       uint64_t step = (uint64_t)start_parity + (uint64_t)k;  // only the parity matters
       enqueue_step(d, step == 0 ? 2 : step, d->u_in, macro_last && k == kGraphChunk - 1, false, false,
-                   false);
+                   STEP_CAPTURED);
     }
     if (cudaStreamEndCapture(cap, &graph) == cudaSuccess && graph) {
       if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) exec = nullptr;
@@ -738,21 +740,26 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
     return PW_ERR_INVALID;
   }
   uint64_t k = 0;
-  const bool early = !d->shared;
+  const StepLaunch how = d->shared ? STEP_BESIDE : STEP_EARLY;
   // ramped steps, one launch each with its own inlet speed
   while (k < count && d->desc.ramp_steps > 0 && d->steps < d->desc.ramp_steps) {
     uint64_t step = d->steps + 1;
     enqueue_step(d, step, ramp_speed(d, step), write_macro_on_last && k == count - 1,
-                 write_macro_on_last && k + 2 == count, k > 0, early);
+                 write_macro_on_last && k + 2 == count, k > 0, how);
     d->steps++;
     k++;
   }
   // full-speed steps: graph chunks when the domain is small enough to be launch bound.
   // A step of one launch needs none (its successor is launched while it runs; in a graph
-  // the 128x64x64 FP32 vehicle's step took as long), and a split step of more than a
+  // the 128x64x64 FP32 vehicle's step took as long) but a small closure domain's, and a split step of more than a
   // million cells is faster without (its side kernels lose their head start in a graph:
   // 192x96x96 FP16 45.9 us a step against 37.9; 128x64x64 24.0 against 28.9).
-  const bool use_graphs = !single_launch(d) && d->cells <= (size_t)(d->split ? 1 : 8) << 20;
+  const bool closure_graphs =
+      d->closure_frag && d->split &&
+      pwclosure_host::closure_long_runs_captured(d->nx, d->ny, d->nz, d->floor_rows, d->edge_own);
+  const bool use_graphs =
+      closure_graphs || (!single_launch(d) && d->cells <= (size_t)(d->split ? 1 : 8) << 20);
+  uint64_t past_graphs = 0;  // a captured step clears no guard flag for the one behind it
   while (use_graphs && count - k >= (uint64_t)kGraphChunk) {
     int macro_last = write_macro_on_last && (count - k == (uint64_t)kGraphChunk);
     cudaGraphExec_t g = graph_for(d, (int)((d->steps + 1) & 1), macro_last);
@@ -760,11 +767,12 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
     if (cudaGraphLaunch(g, d->stream) != cudaSuccess) { cudaGetLastError(); break; }
     d->steps += kGraphChunk;
     k += kGraphChunk;
+    past_graphs = k;
   }
   for (; k < count; k++) {
     uint64_t step = d->steps + 1;
-    enqueue_step(d, step, d->u_in, write_macro_on_last && k == count - 1, write_macro_on_last && k + 2 == count, k > 0,
-                 early);
+    enqueue_step(d, step, d->u_in, write_macro_on_last && k == count - 1, write_macro_on_last && k + 2 == count,
+                 k > 0 && k != past_graphs, how);
     d->steps++;
   }
   PW_TRY(cudaGetLastError());

@@ -78,10 +78,13 @@ void launch_closure_step(const pw::StepParams &p, int storage, int op, bool odd,
 // The same step for periodic faces in the cell-pair form, one launch: every row's
 // plain cells two per thread with the network on the block's two 128-cell tiles, and
 // the listed edge cells and the floor layer in blocks of their own; taken: a counter that
-// is zero between steps; early: the step may start while the one before it ends.
+// is zero between steps; early: the step may start while the one before it ends.  With side
+// the edge cells and the floor layer run in kernels of their own on its stream.
 void launch_closure_pairs(const pw::StepParams &p, int storage, int op, bool odd, const uint32_t *frag,
                           const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken, bool early,
-                          cudaStream_t s);
+                          cudaStream_t s, const pwfast::SideStream *side = nullptr);
+// Whether a long run of such steps is faster captured, with side, than launched early.
+bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int floor_rows, uint32_t count);
 int wall_distance_of(const uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *out, cudaStream_t s);
 const uint32_t *fragments(const pw_closure *c);
 }

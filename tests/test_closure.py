@@ -333,3 +333,59 @@ def test_trained_closure_beats_smagorinsky_on_held_out_data():
     assert np.isfinite(cs.macros()).all()
     c.destroy()
     s.destroy()
+
+
+# sizes whose long runs are captured (64 steps a graph) and, the last, one past the line;
+# 65 and 129 steps leave one step behind the graphs
+@pytest_gpu
+@pytest.mark.parametrize("precision,layout", [("f32", (64, 32, 32)), ("f16", (33, 17, 17)), ("f32", (72, 36, 36))])
+@pytest.mark.parametrize("count", [64, 65, 129])
+def test_long_closure_runs_equal_single_steps(precision, layout, count):
+    from pocketwind_gb300 import geometry, meshes, solver
+    net = _closure(_rand_params(9))
+    grid = geometry.voxelize(meshes.icosphere([n / 2.2 for n in layout], min(layout) / 5, 3), None, layout, True)
+    got = []
+    for calls in ([1] * count, [count]):
+        s = solver.GpuSolver.create(layout, grid, solver.SolverParams(tau0=0.56, u_in=0.05, les=True, operator="reg",
+                                                                      precision=precision))
+        net.attach(s)
+        s.inject_nan()
+        s.step(1, True)
+        assert s.guard_unstable()
+        s.reset()
+        for k, n in enumerate(calls):
+            s.step(n, k + 1 == len(calls))
+        assert not s.guard_unstable()
+        s.encode_force()
+        f = s.read_force()
+        got.append((s.populations_raw().view(np.uint8), s.macros(), (f.fx, f.fy, f.fz)))
+        s.destroy()
+    net.destroy()
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1], got[1][1])
+    assert got[0][2] == got[1][2]
+
+
+@pytest_gpu
+def test_long_closure_runs_of_small_domains_are_captured():
+    """A step of 256 in a call costs less than one of 8 in calls of 8 (64x32x32: 12.4 and 14.3
+    us; launched early 13.7)."""
+    import time
+    from pocketwind_gb300 import cases, solver
+    v = cases.vehicle_case(64)
+    s = solver.GpuSolver.create(v.layout, v.grid(), v.params("f32"))
+    net = _closure(_rand_params(9))
+    net.attach(s)
+    best = []
+    for count in (8, 256):
+        times = []
+        for _ in range(40):
+            t = time.perf_counter()
+            for _ in range(256 // count):
+                s.step(count)
+            s.guard_unstable()
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+    s.destroy()
+    net.destroy()
+    assert best[1] < 0.95 * best[0], best
