@@ -331,9 +331,9 @@ PW_API int pw_closure_attach(pw_domain *dom, const pw_closure *c);
 PW_API int pw_time_steps(pw_domain *dom, uint64_t count, float *ms);
 /* Queue `count` steps (no graphs) with CUDA events around each launch class and
    sum their device times: kernel_ms[0] the plain-cell kernel, [1] its seam-row
-   variant (odd steps), [2] the edge-cell kernel.  Outside the fast build's
-   one-cell-per-thread path the whole step counts as [0].  No counterpart in the
-   reference (a measurement aid). */
+   variant (odd steps), [2] the edge-cell kernel.  A step of one launch, and any
+   outside the fast build's one-cell-per-thread path, counts whole as [0].  No
+   counterpart in the reference (a measurement aid). */
 PW_API int pw_profile_steps(pw_domain *dom, uint64_t count, float kernel_ms[3]);
 
 /* ---------------------------------------------------------------- tracers */

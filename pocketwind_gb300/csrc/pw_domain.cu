@@ -936,6 +936,7 @@ int pw_domain_share(pw_domain *d, int shared) {
 int pw_profile_steps(pw_domain *d, uint64_t count, float kernel_ms[3]) {
   if (!alive(d) || !kernel_ms) { set_error("NULL argument"); return PW_ERR_INVALID; }
   kernel_ms[0] = kernel_ms[1] = kernel_ms[2] = 0.0f;
+  const bool whole = !d->split || single_launch(d);  // a step's time is [0]
   constexpr int kBatch = 32;
   cudaEvent_t ev[kBatch][6];
   int made = 0;
@@ -948,19 +949,19 @@ int pw_profile_steps(pw_domain *d, uint64_t count, float kernel_ms[3]) {
       const uint64_t step = d->steps + 1;
       pw::StepParams p = params_for(d, step, ramp_speed(d, step), 0);
       const bool odd = (step & 1) != 0;
-      if (d->split && !d->closure_frag) {
+      if (!whole) {
         pwfast::launch_step_split(p, d->desc.storage, d->desc.op, d->desc.les, odd, d->plain_grid, d->edges,
                                   d->edge_own, d->stream, ev[b]);
       } else {
         cudaEventRecord(ev[b][0], d->stream);
-        enqueue_step(d, step, ramp_speed(d, step), 0);
+        enqueue_step(d, step, ramp_speed(d, step), 0, false, false, d->shared ? STEP_BESIDE : STEP_EARLY);
         for (int m = 1; m < 6; m++) cudaEventRecord(ev[b][m], d->stream);
       }
       d->steps++;
     }
     e = cudaEventSynchronize(ev[n - 1][5]);
     for (int b = 0; b < n && e == cudaSuccess; b++) {
-      for (int c = 0; c < 3 && e == cudaSuccess; c++) {
+      for (int c = 0; c < (whole ? 1 : 3) && e == cudaSuccess; c++) {
         float t = 0.0f;
         e = cudaEventElapsedTime(&t, ev[b][2 * c], ev[b][2 * c + 1]);
         kernel_ms[c] += t;

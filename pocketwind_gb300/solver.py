@@ -153,7 +153,8 @@ class GpuSolver:
 
     def profile_steps(self, count: int) -> tuple:
         """Summed device milliseconds of the plain-cell, seam-row and edge-cell
-        kernels over ``count`` steps (CUDA events around each launch)."""
+        kernels over ``count`` steps (CUDA events around each launch); a step of one
+        launch counts whole as the first."""
         ms = (C.c_float * 3)()
         _lib.check(_lib.load().pw_profile_steps(self._live(), int(count), ms), "profile_steps")
         return tuple(ms)

@@ -739,3 +739,23 @@ def test_shared_domain_stores_the_same_values(layout, precision):
         assert np.array_equal(got[0][0], other[0])
         assert np.array_equal(got[0][1], other[1])
         assert got[0][2:] == other[2:]
+
+
+def test_profiled_steps_of_one_launch_count_whole():
+    """profile_steps times what step() runs: a step of one launch as the first kernel, one
+    after another the split step's three; the state goes on as by step()."""
+    from pocketwind_gb300 import cases
+    case = cases.vehicle_case(64)
+    grid = case.grid()
+    G, S = _pw()
+    a, b = (S.GpuSolver.create(case.layout, grid, case.params("f32")) for _ in range(2))
+    ms = a.profile_steps(41)
+    b.step(41)
+    assert a.step_count == 41 and ms[0] > 0.9 * sum(ms), ms
+    assert np.array_equal(a.populations(), b.populations())
+    a.destroy()
+    b.destroy()
+    split = make_solver(*blob_grid(), precision="f16", lateral="free-slip")
+    ms = split.profile_steps(40)
+    assert min(ms) > 0 and ms[0] < 0.9 * sum(ms), ms
+    split.destroy()
