@@ -320,3 +320,39 @@ def test_members_of_few_cells_share_the_persistent_launches(layout, own):
     batch.tune(2)
     assert own or not batch.own_launches
     batch.destroy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [(48, 24, 24), (49, 25, 23)])
+@pytest.mark.parametrize("precision", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("form", FORMS)
+def test_persistent_members_equal_solo_runs(form, precision, layout):
+    """Members of few cells (persistent launches; 50 steps from a captured graph) hold the bits of
+    the same domain stepped alone, but a 16-bit floor's layer, which a solo step takes in
+    closed form (test_floor_kernel_matches_the_general_path)."""
+    other = tuple(n - 8 for n in layout)
+    a = _stepped_in_batch([layout, other], precision, form)
+    assert not a[3]
+    s = _form_member(layout, precision, **FORMS[form])
+    for n in (1, 6, 50):
+        s.step(n, True)
+    s.encode_force()
+    f = s.read_force()
+    if precision != "f32" and "floor" in form and layout[0] % 2 == 0:
+        assert _l2_err(a[1][:, 1:], s.macros()[:, 1:]) < (2e-3 if precision == "f16" else 1e-2)
+    else:
+        assert np.array_equal(a[0], s.populations_raw().view(np.uint8))
+        assert np.array_equal(a[1], s.macros())
+        assert a[2] == (f.fx, f.fy, f.fz)
+    s.destroy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["trt", "reg floor", "reg les slip"])
+def test_persistent_batch_is_deterministic(form):
+    """As test_batch_step_is_deterministic, by the two concurrent persistent launches."""
+    layouts = [(48, 24, 24), (36, 20, 22), (64, 30, 20)]
+    a, b = (_stepped_in_batch(layouts, "f16", form) for _ in range(2))
+    assert not a[3]
+    assert np.array_equal(a[0], b[0])
+    assert a[2] == b[2]

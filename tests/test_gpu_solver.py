@@ -716,7 +716,7 @@ def test_domain_leaves_the_stream_ordered_pool_alone():
 
 
 @pytest.mark.parametrize("precision", ["f32", "f16", "bf16"])
-@pytest.mark.parametrize("layout", [(64, 32, 32), (65, 33, 32), (160, 90, 80), (161, 91, 81)])
+@pytest.mark.parametrize("layout", [(64, 32, 32), (65, 33, 32), (128, 80, 64), (160, 90, 80), (161, 91, 81)])
 def test_shared_domain_stores_the_same_values(layout, precision):
     """A domain that shares the GPU runs other block forms, above a million cells the split
     step; the codes, macros, guard and drag are the same bits, also when that changes on the way."""
@@ -739,6 +739,55 @@ def test_shared_domain_stores_the_same_values(layout, precision):
         assert np.array_equal(got[0][0], other[0])
         assert np.array_equal(got[0][1], other[1])
         assert got[0][2:] == other[2:]
+
+
+# nx odd, 16-bit storage, ny even and odd: the pairs over a plane's cells beside reflecting
+# seam rows, interpolated walls and the wall model over a floor
+@pytest.mark.parametrize("layout", [(49, 24, 24), (47, 25, 23)])
+@pytest.mark.parametrize("precision", ["f16", "bf16"])
+@pytest.mark.parametrize("kw", [dict(lateral="free-slip"), dict(lateral="free-slip", les=True, op="reg"),
+                                dict(walls="bouzidi"), dict(walls="bouzidi", les=True, op="reg"),
+                                dict(les=True, op="reg", floor=True), dict(les=True, floor=True)],
+                         ids=["slip", "slip reg les", "bouzidi", "bouzidi reg les", "reg floor", "trt floor"])
+def test_odd_rows_in_every_form_within_reference_rounding_noise(kw, precision, layout):
+    """The bound of test_fast_16bit_within_reference_rounding_noise."""
+    from pocketwind_gb300 import meshes
+    kw = dict(kw)
+    floor = kw.pop("floor", False)
+    grid = O.voxelize(meshes.icosphere((12.3, 11.62, 12.41), 4, 3).positions, None, layout, floor,
+                      link_fractions=kw.get("walls") == "bouzidi")
+    fast = make_solver(grid.geometry, grid.boundary_cells, layout, tau0=0.56, u_in=0.05, precision=precision, **kw)
+    ref32, ref16 = (O.Wgsl32(*layout, 0.56, 0.05, grid.geometry, grid.boundary_cells, storage=st, **kw)
+                    for st in ("f32", precision))
+    fast.step(16, True)
+    for k in range(16):
+        ref32.step(0.05, k == 15)
+        ref16.step(0.05, k == 15)
+    want = ref32.populations()
+    err, ref_err = norm_err(fast.populations(), want), norm_err(ref16.populations(), want)
+    assert np.isfinite(err) and err <= 2 * ref_err, (err, ref_err)
+    fast.destroy()
+
+
+@pytest.mark.parametrize("layout", [(49, 24, 24), (47, 25, 23)])
+@pytest.mark.parametrize("precision,op,les,lateral", [
+    ("f16", "trt", False, "periodic"), ("f16", "reg", True, "periodic"), ("bf16", "trt", True, "periodic"),
+    ("f16", "trt", False, "free-slip"), ("bf16", "reg", True, "free-slip"), ("f32", "trt", False, "periodic")])
+def test_odd_rows_are_deterministic(precision, op, les, lateral, layout):
+    """As test_fast_step_is_deterministic: pairs that run over a row's end read and store half
+    words beside their neighbours'."""
+    from pocketwind_gb300 import meshes
+    G, S = _pw()
+    grid = G.voxelize(meshes.icosphere((16, 12.3, 11.4), 5, 3), None, layout, False)
+    runs = []
+    for _ in range(4):
+        s = S.GpuSolver.create(layout, grid, S.SolverParams(tau0=0.56, u_in=0.05, les=les, operator=op,
+                                                            precision=precision, lateral=lateral))
+        s.step(60, True)
+        runs.append(s.populations_raw().view(np.uint8).copy())
+        s.destroy()
+    for r in runs[1:]:
+        assert np.array_equal(r, runs[0])
 
 
 def test_profiled_steps_of_one_launch_count_whole():
