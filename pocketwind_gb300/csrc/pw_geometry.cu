@@ -78,52 +78,57 @@ Grid::~Grid() {
 
 // ------------------------------------------------------------------ pinned slots
 namespace {
-struct PinnedSlab {
-  char *base;
-  uint64_t used;  // a bit a slot
-};
 constexpr size_t kSlabSlots = 64;
+// A slab's head, in its own first slot: no container to grow, so nothing here throws
+// through a C entry.
+struct PinnedSlab {
+  PinnedSlab *next;
+  uint64_t used;  // a bit a slot; bit 0, the head's own, is always set
+  bool empty() const { return used == 1u; }
+  char *slot(int k) { return reinterpret_cast<char *>(this) + (size_t)k * kPinnedSlot; }
+};
+static_assert(sizeof(PinnedSlab) <= kPinnedSlot, "the head fits a slot");
 std::mutex g_pinned_lock;
-std::vector<PinnedSlab> g_pinned;
+PinnedSlab *g_pinned = nullptr;
 }  // namespace
 
 void *pinned_acquire() {
   std::lock_guard<std::mutex> hold(g_pinned_lock);
-  PinnedSlab *slab = nullptr;
-  for (PinnedSlab &s : g_pinned)
-    if (~s.used) { slab = &s; break; }
+  PinnedSlab *slab = g_pinned;
+  while (slab && !~slab->used) slab = slab->next;
   if (!slab) {
     void *p = nullptr;
     if (cudaHostAlloc(&p, kSlabSlots * kPinnedSlot, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
-    g_pinned.push_back(PinnedSlab{static_cast<char *>(p), 0});
-    slab = &g_pinned.back();
+    slab = static_cast<PinnedSlab *>(p);
+    *slab = PinnedSlab{g_pinned, 1u};
+    g_pinned = slab;
   }
   const int k = __builtin_ctzll(~slab->used);
   slab->used |= 1ull << k;
-  void *slot = slab->base + (size_t)k * kPinnedSlot;
-  std::memset(slot, 0, kPinnedSlot);
-  return slot;
+  std::memset(slab->slot(k), 0, kPinnedSlot);
+  return slab->slot(k);
 }
 
 void pinned_release(void *slot) {
   std::lock_guard<std::mutex> hold(g_pinned_lock);
   bool other_empty = false;
-  size_t at = g_pinned.size();
-  for (size_t i = 0; i < g_pinned.size(); i++) {
-    const ptrdiff_t off = static_cast<char *>(slot) - g_pinned[i].base;
-    if (off >= 0 && off < (ptrdiff_t)(kSlabSlots * kPinnedSlot)) {
-      g_pinned[i].used &= ~(1ull << (off / (ptrdiff_t)kPinnedSlot));
-      at = i;
-    } else if (!g_pinned[i].used) {
+  PinnedSlab **own = nullptr;
+  for (PinnedSlab **at = &g_pinned; *at; at = &(*at)->next) {
+    const ptrdiff_t off = static_cast<char *>(slot) - (*at)->slot(0);
+    if (off > 0 && off < (ptrdiff_t)(kSlabSlots * kPinnedSlot)) {
+      (*at)->used &= ~(1ull << (off / (ptrdiff_t)kPinnedSlot));
+      own = at;
+    } else if ((*at)->empty()) {
       other_empty = true;
     }
   }
-  if (at < g_pinned.size() && !g_pinned[at].used && other_empty) {
-    cudaFreeHost(g_pinned[at].base);
-    g_pinned.erase(g_pinned.begin() + (ptrdiff_t)at);
+  if (own && (*own)->empty() && other_empty) {
+    PinnedSlab *gone = *own;
+    *own = gone->next;
+    cudaFreeHost(gone);
   }
 }
 

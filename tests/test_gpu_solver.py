@@ -808,3 +808,36 @@ def test_profiled_steps_of_one_launch_count_whole():
     ms = split.profile_steps(40)
     assert min(ms) > 0 and ms[0] < 0.9 * sum(ms), ms
     split.destroy()
+
+
+def test_many_domains_hold_their_own_results():
+    """130 domains (their pinned slots fill two slabs and begin a third), half of them given
+    back in between and taken anew: every drag is its own domain's."""
+    from pocketwind_gb300 import meshes
+    G, S = _pw()
+    layout = (16, 8, 8)
+    grid = G.voxelize(meshes.icosphere((5.2, 4.1, 3.9), 2.2, 2), None, layout, False)
+
+    def make(k):
+        s = S.GpuSolver.create(layout, grid, S.SolverParams(tau0=0.8, u_in=0.01 + 0.0004 * (k % 65)))
+        s.step(4, True)
+        return s
+
+    def drag(s):
+        s.encode_force()
+        return s.read_force().fx
+
+    alone = make(7)
+    want = drag(alone)
+    alone.destroy()
+    many = [make(k) for k in range(130)]
+    for k in range(0, 130, 2):
+        many[k].destroy()
+        many[k] = make(k)
+    for s in many:
+        s.encode_force()
+    got = [s.read_force().fx for s in many]
+    assert got[7] == got[72] == want
+    assert got[:65] == got[65:] and len(set(got)) == 65
+    for s in many[::-1]:
+        s.destroy()
