@@ -381,13 +381,6 @@ int queue_steps(pw_batch *b, uint64_t count, int macro_last) {
   return PW_OK;
 }
 
-int max_blocks() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, sms);
-}
-
 }  // namespace
 
 extern "C" {
@@ -444,7 +437,7 @@ int pw_batch_create(pw_domain *const *members, uint32_t count, pw_batch **out) {
   // the host's, and 99 by the persistent ones from a graph; 32 of 72x36x36 (93 K) 90 and 114.
   b->can_own = b->can_own && cells >= (uint64_t)count * (80u << 10);
   b->own = b->can_own;
-  b->sms = (unsigned)max_blocks();
+  b->sms = multiprocessors();
   b->blocks = b->sms * 32u;  // with 8 rows an item within 4% of what tuning finds (4 and 4: half the rate)
   auto fail = [&](int rc) {
     pw_batch_destroy(b);
@@ -556,7 +549,7 @@ int pw_batch_time_steps(pw_batch *b, uint64_t count, float *ms) {
 int pw_batch_tune(pw_batch *b, uint32_t trial_steps, pw_batch_tuning *out) {
   if (!b || trial_steps == 0) { set_error("The batch handle is NULL or the trial has no steps."); return PW_ERR_INVALID; }
   trial_steps += trial_steps & 1u;
-  const unsigned sms = (unsigned)max_blocks();
+  const unsigned sms = multiprocessors();
   const unsigned grid_mult[] = {2, 4, 8, 16, 32};
   const uint32_t row_opts[] = {8, 16, 32, 64};
   b->own = false;

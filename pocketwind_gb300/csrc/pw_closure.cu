@@ -44,20 +44,6 @@ using namespace pwhost;
 using pw::StepParams;
 using namespace pwcl;
 
-namespace pwclosure_host {
-// Multiprocessors of the current device, cached per device (1 when unknown).
-static int sm_count() {
-  static int sms[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); dev = 0; }
-  if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    sms[dev] = 1;
-  }
-  return std::max(sms[dev], 1);
-}
-}  // namespace pwclosure_host
-
 namespace {
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -1229,7 +1215,7 @@ namespace {
 
 // Blocks of a training pass: one an SM, fewer for a batch of fewer groups of 32.
 uint32_t train_blocks(uint32_t batch) {
-  return std::min((batch + 31u) / 32u, (uint32_t)pwclosure_host::sm_count());
+  return std::min((batch + 31u) / 32u, multiprocessors());
 }
 
 int ensure_partials(pw_closure *c, uint32_t blocks) {
@@ -1256,7 +1242,7 @@ void launch_closure_step(const StepParams &p, int storage, int op, bool odd, dim
                          const uint8_t *wall, cudaStream_t s) {
   const dim3 blk(32, 4);
   const uint32_t tiles = grid.x * grid.y * grid.z;
-  const unsigned g = (unsigned)std::min<uint32_t>(tiles, 4u * (uint32_t)sm_count());
+  const unsigned g = (unsigned)std::min<uint32_t>(tiles, 4u * multiprocessors());
 #define PW_CL_LAUNCH(ST, OPV)                                                                  \
   do {                                                                                        \
     if (odd) closure_step<ST, OPV, true><<<g, blk, 0, s>>>(p, frag, wall, grid.x, grid.y);    \
@@ -1279,7 +1265,7 @@ static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const 
                                uint32_t row_blocks, const ClosureSide &side, bool early, cudaStream_t s) {
   // the blocks that fit at once: the launch bound's count per SM (registers; 20 KB of
   // shared memory and 64 TMEM columns a block leave room for more)
-  const uint32_t tiles = runs * row_blocks * p.nz, walk = std::min(tiles, (uint32_t)BLOCKS * (uint32_t)sm_count());
+  const uint32_t tiles = runs * row_blocks * p.nz, walk = std::min(tiles, (uint32_t)BLOCKS * multiprocessors());
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(side.edge + side.floor + walk);
   cfg.blockDim = dim3(32, 4);
@@ -1314,7 +1300,7 @@ static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const 
   }
   ClosureSide side{list, count, (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS, 0u, taken};
   if (ST != pw::STORE_F32 && p.floor_rows && p.ny >= 3u) side.floor = runs * ((p.ny - 2u + 3u) / 4u);
-  if ((uint64_t)runs * row_blocks * p.nz + side.edge + side.floor <= (uint64_t)PW_CLOSURE_FEW_BLOCKS * sm_count())
+  if ((uint64_t)runs * row_blocks * p.nz + side.edge + side.floor <= (uint64_t)PW_CLOSURE_FEW_BLOCKS * multiprocessors())
     closure_pairs_step<ST, OP, ODD, PW_CLOSURE_FEW_BLOCKS>(p, frag, wall, runs, row_blocks, side, early, s);
   else
     closure_pairs_step<ST, OP, ODD, PW_CLOSURE_PAIR_BLOCKS>(p, frag, wall, runs, row_blocks, side, early, s);
@@ -1331,7 +1317,7 @@ static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const 
 // own the early launches are the faster ones at any size (FP16 64x32x32 16.1 and 16.3).
 bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int floor_rows, uint32_t count) {
   if (floor_rows && ny >= 3u) return false;
-  const uint64_t tiles = (uint64_t)((nx + 63u) / 64u) * ((ny + 3u) / 4u) * nz, sms = (uint64_t)sm_count();
+  const uint64_t tiles = (uint64_t)((nx + 63u) / 64u) * ((ny + 3u) / 4u) * nz, sms = (uint64_t)multiprocessors();
   const uint64_t edge = (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS;
   return 5u * tiles <= (8u * edge < sms ? 25u : 21u) * sms;
 }

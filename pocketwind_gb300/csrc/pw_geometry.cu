@@ -17,6 +17,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstring>
@@ -24,6 +25,7 @@
 #include <vector>
 
 #include "pw_internal.h"
+#include "pw_launch.h"
 
 namespace pwhost {
 
@@ -69,6 +71,21 @@ static cudaError_t tmp_alloc(void *p, size_t bytes, cudaStream_t s) {
 }
 static void tmp_free(void *p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
+}
+
+uint32_t multiprocessors() {
+  static std::atomic<int> counts[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); dev = 0; }
+  int n = counts[dev].load(std::memory_order_relaxed);
+  if (!n) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 1;
+    }
+    counts[dev].store(n, std::memory_order_relaxed);
+  }
+  return (uint32_t)n;
 }
 
 Grid::~Grid() {
@@ -674,7 +691,7 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
   }
   GridInfo got{};
   double *hits = nullptr;
-  // one warp a group of 32 triangles, or as many as fill the GPU's 152 SMs with 16
+  // one warp a group of 32 triangles, or as many as fill the SMs with 16
   const uint32_t groups = (ntri + 31u) / 32u;
   cudaError_t e = tmp_alloc(votes_out, (cells + 3) / 4 * 4, s);
   uint8_t *votes = *votes_out;
@@ -685,7 +702,7 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
   HeavyGroup *heavy = reinterpret_cast<HeavyGroup *>(columns);
   uint32_t *count = reinterpret_cast<uint32_t *>(columns + notes), *offset = count + ncol;
   int rc = e == cudaSuccess ? PW_OK : cuda_status(e, "voxelize columns");
-  const uint32_t slices = std::max(1u, std::min(1024u, 152u * 16u / groups));
+  const uint32_t slices = std::max(1u, std::min(1024u, multiprocessors() * 16u / groups));
   const unsigned rblocks = (unsigned)(((uint64_t)groups * slices + kRasterThreads / 32 - 1) / (kRasterThreads / 32));
   if (rc == PW_OK) {
     cudaMemsetAsync(votes, 0, (cells + 3) / 4 * 4, s);
@@ -698,7 +715,7 @@ static int vote_mesh(const float *d_mesh, uint32_t ntri, uint32_t nx, uint32_t n
   const uint32_t noted = heavy_groups(got.heavy[which]);
   const unsigned long long pieces = heavy_pieces(got.heavy[which]);
   const unsigned hblocks = (unsigned)std::min<unsigned long long>((pieces + kRasterThreads / 32 - 1) / (kRasterThreads / 32),
-                                                                  152u * 16u);
+                                                                  16ull * multiprocessors());
   if (rc == PW_OK && noted && !got.nonfinite) {  // their hits too, and the columns' offsets anew
     raster_heavy<false><<<hblocks, kRasterThreads, 0, s>>>(d_mesh, ntri, P, heavy, noted, pieces, count, nullptr,
                                                            nullptr);

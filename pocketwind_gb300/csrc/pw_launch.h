@@ -58,6 +58,10 @@ void launch_refresh_edges(const pw::StepParams &p, int odd_layout, int storage, 
                           uint32_t count, cudaStream_t s);
 }
 PW_DECLARE_LAUNCHERS(pwstrict)
+namespace pwhost {
+// Multiprocessors of the current device, asked once per device (1 when unknown).
+uint32_t multiprocessors();
+}
 // The same split step in one launch, blocks by role (pw_step_all.cuh).
 namespace pwall {
 bool step_all_supported(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int op, int les, uint32_t slip);

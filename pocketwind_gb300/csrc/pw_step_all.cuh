@@ -108,7 +108,7 @@ namespace {
 // 192x96x96 31.8 and 30.4; 208x104x104 44.5 and 46.3).  Domains stepped side by side
 // share the SMs and keep the form for large ones.
 constexpr int kPairBlocks = 8, kCellBlocks = 7, kLinearBlocks = 7, kFewBlocks = 4, kMidBlocks = 6;
-constexpr uint32_t kSms = 152, kFewPerSm = 16, kMidPerSmRuns = 32, kMidPerSmPairs = 48;
+constexpr uint32_t kFewPerSm = 16, kMidPerSmRuns = 32, kMidPerSmPairs = 48;
 
 template <int ST, int OP, bool LES, Plain FORM, int BLOCKS>
 void launch_grid(const StepParams &p, bool odd, const uint32_t *list, uint32_t count, const SideBlocks &w, dim3 grid,
@@ -142,7 +142,7 @@ void launch4(const StepParams &p, bool odd, const uint32_t *list, uint32_t count
   if (p.clear_status && w.slices == 0u) w.slices = 1u;  // its first thread clears the flag
   const dim3 grid(gx, gy, p.nz - 2u * off + w.slices);
   constexpr int kMany = FORM == RUNS ? kCellBlocks : (pairs ? kPairBlocks : kLinearBlocks);
-  const uint64_t per_sm = (uint64_t)slice * (p.nz - 2u * off) / kSms;
+  const uint64_t per_sm = (uint64_t)slice * (p.nz - 2u * off) / pwhost::multiprocessors();
   if (early && per_sm < kFewPerSm) {
     launch_grid<ST, OP, LES, FORM, kFewBlocks>(p, odd, list, count, w, grid, s, early);
     return;
