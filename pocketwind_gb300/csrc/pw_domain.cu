@@ -655,6 +655,7 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   a.want((void **)&d->status_dev, 16);
   a.want((void **)&d->tiles_taken, sizeof(uint32_t));
   a.want((void **)&d->totals_dev, 4 * sizeof(double));
+  prepare_pool();
   if (e == cudaSuccess) e = a.alloc(&d->arena);
   if (e == cudaSuccess) {
     char *slot = static_cast<char *>(pinned_acquire());

@@ -56,18 +56,31 @@ int cuda_status(cudaError_t e, const char *what) {
 // one never waits for the whole device, and the pool keeps up to 256 MB mapped
 // between calls.
 static cudaError_t tmp_alloc(void *p, size_t bytes, cudaStream_t s) {
-  static bool pool_set = false;
-  if (!pool_set) {
-    int dev = 0;
-    cudaMemPool_t pool;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-      uint64_t keep = 256ull << 20;
-      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
-    cudaGetLastError();
-    pool_set = true;
-  }
+  prepare_pool();
   return cudaMallocAsync(reinterpret_cast<void **>(p), bytes, s);
+}
+
+// The pool takes its place in the address space here, on a stream of its own.
+void prepare_pool() {
+  static std::mutex lock;
+  static bool done[64];
+  int dev = 0;
+  std::lock_guard<std::mutex> hold(lock);
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev]) { cudaGetLastError(); return; }
+  done[dev] = true;
+  cudaMemPool_t pool;
+  cudaStream_t s;
+  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+    uint64_t keep = 256ull << 20;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess) {
+    void *p = nullptr;
+    if (cudaMallocAsync(&p, 1024, s) == cudaSuccess) cudaFreeAsync(p, s);
+    cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+  }
+  cudaGetLastError();
 }
 static void tmp_free(void *p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);

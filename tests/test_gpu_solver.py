@@ -841,3 +841,25 @@ def test_many_domains_hold_their_own_results():
     assert got[:65] == got[65:] and len(set(got)) == 65
     for s in many[::-1]:
         s.destroy()
+
+
+def test_first_domain_sets_the_pool_up():
+    """In a process that creates a domain before it voxelizes, the stream-ordered pool is set up
+    (CU_MEMPOOL_ATTR_RELEASE_THRESHOLD, 4) ahead of the domain's memory."""
+    import subprocess
+    import sys
+    code = """
+import ctypes as C
+from tests.shapes import blob_grid
+from tests.test_gpu_solver import make_solver
+s = make_solver(*blob_grid())
+cuda = C.CDLL("libcuda.so.1")
+pool, keep = C.c_void_p(), C.c_uint64()
+assert cuda.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+assert cuda.cuMemPoolGetAttribute(pool, 4, C.byref(keep)) == 0
+print(keep.value)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stderr
+    assert int(out.stdout.split()[-1]) == 256 << 20
