@@ -429,13 +429,15 @@ int pw_batch_create(pw_domain *const *members, uint32_t count, pw_batch **out) {
     const MemberView v = member_view(members[m]);
     b->can_own = b->can_own && v.one_launch;
     ((v.nx & 1u) ? odd : even) = true;
-    cells += (uint64_t)v.nx * v.ny * v.nz;
+    cells += (uint64_t)((v.nx + 63u) / 64u * 64u) * v.ny * v.nz;
   }
   if (b->storage != pw::STORE_F32 && odd && even) b->can_own = false;
-  // Below 80 K cells a member its launch takes the host as long as its step the GPU: 64
-  // tunnels of 64x32x32 (65 K cells) FP16 157 us a step by their own launches, 151 of them
-  // the host's, and 99 by the persistent ones from a graph; 32 of 72x36x36 (93 K) 90 and 114.
-  b->can_own = b->can_own && cells >= (uint64_t)count * (80u << 10);
+  // The host queues a member's own step in 2.5 us; the persistent launches, which walk rows of
+  // 64 cells, take 1.5 us (16-bit) or 2.3 (FP32) for 64 K cells of such rows.  So the line
+  // lies at 96 K and 72 K of them a member.  Persistent and own, 64 members a step: FP16
+  // 64x32x32 103 and 162 us, 64x40x40 (100 K) 157 and 162, with a floor 175 and 164, 65x33x33
+  // (136 K) 221 and 163; FP32 64x32x32 151 and 162, 64x40x32 (80 K) 186 and 171.
+  b->can_own = b->can_own && cells >= (uint64_t)count * ((b->storage == pw::STORE_F32 ? 72u : 96u) << 10);
   b->own = b->can_own;
   b->sms = multiprocessors();
   b->blocks = b->sms * 32u;  // with 8 rows an item within 4% of what tuning finds (4 and 4: half the rate)

@@ -309,12 +309,14 @@ def test_mixed_widths_keep_one_form(precision):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("layout,own", [((64, 32, 32), False), ((80, 32, 31), False), ((80, 32, 32), True),
-                                        ((72, 36, 36), True)])
-def test_members_of_few_cells_share_the_persistent_launches(layout, own):
-    """The line is 80 K cells a member; below it tuning keeps the persistent launches too."""
+@pytest.mark.parametrize("precision,layout,own", [
+    ("f16", (64, 32, 32), False), ("f16", (64, 48, 31), False), ("f16", (64, 48, 32), True), ("f16", (65, 25, 32), True),
+    ("f32", (64, 32, 32), False), ("f32", (64, 36, 31), False), ("f32", (64, 36, 32), True), ("bf16", (33, 40, 32), False)])
+def test_members_of_few_cells_share_the_persistent_launches(precision, layout, own):
+    """The line is 96 K cells a member (FP32 72 K) in rows of 64; below it tuning keeps the
+    persistent launches too."""
     from pocketwind_gb300.batch import Batch
-    members = [_form_member(layout, "f16") for _ in range(2)]
+    members = [_form_member(layout, precision) for _ in range(2)]
     batch = Batch(members)
     assert batch.own_launches == own
     batch.tune(2)
