@@ -295,7 +295,17 @@ pw::StepParams params_for(const pw_domain *d, uint64_t step, float u_in, int wri
 // early, as when one after another, 173.7, 125.7 and 124.1 (blocks that wait for their
 // step hold the places of the other domains').
 constexpr size_t kSharedOneLaunch = (size_t)1 << 20;
-bool split_in_one(const pw_domain *d) { return d->one_launch && !(d->shared && d->cells > kSharedOneLaunch); }
+// Large binary32 domains of the regularized operator are faster split too, as in 16 bits
+// (step_all_supported).  One launch and split: with LES and a floor 225x113x112 85.1 and 85.2
+// us, 240x120x120 98.9 and 98.1, 399x200x200 423 and 416, 512x256x256 815 and 807; without LES
+// 288x144x144 159.5 and 160.4, 321x160x161 228.9 and 227.1, 399x200x200 420 and 415.  With TRT
+// one launch is the faster at any size (399x200x200 LES 425 and 432).
+constexpr size_t kRegLesOneLaunch = (size_t)3 << 20, kRegOneLaunch = (size_t)8 << 20;
+bool split_in_one(const pw_domain *d) {
+  if (!d->one_launch || (d->shared && d->cells > kSharedOneLaunch)) return false;
+  return d->desc.storage != PW_STORE_F32 || d->desc.op != PW_OP_REG ||
+         d->cells <= (d->desc.les ? kRegLesOneLaunch : kRegOneLaunch);
+}
 
 // Whether a step is one launch (the split step in that form, the closure's cell pairs).
 bool single_launch(const pw_domain *d) { return d->split && (split_in_one(d) || d->closure_frag); }

@@ -8,8 +8,9 @@ extern template void launch_storage<STORE_F16>(const StepParams &, int, int, boo
 extern template void launch_storage<STORE_BF16>(const StepParams &, int, int, bool, const uint32_t *, uint32_t,
                                                 cudaStream_t, bool);
 
-// Whether a domain's steps run in one launch.  Binary32 storage: always (the vehicle
-// at 64^2 x 128 23.4 us before and 15.0 now, at 256^2 x 512 795 and 794).  16-bit cell
+// Whether a domain's steps may run in one launch.  Binary32 storage: always (the vehicle
+// at 64^2 x 128 23.4 us before and 15.0 now; a large domain of the regularized operator that
+// steps on its own is split, pw_domain.cu's split_in_one).  16-bit cell
 // pairs up to 3.7 M cells with LES, 2.6 M without (split and one launch, by eight steps:
 // FP16 REG LES 224x112x112 55.5 and 54.3 us, 240x120x120 64.1 and 63.5, 256x128x128 74.3
 // and 74.2, BF16 there 73.0 and 74.1, 320x160x160 136.2 and 139.6; FP16 TRT 224x112x112

@@ -863,3 +863,26 @@ print(keep.value)
     out = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stderr
     assert int(out.stdout.split()[-1]) == 256 << 20
+
+
+# the lines of binary32 steps: REG with LES one launch up to 3 M cells and without up to 8 M,
+# TRT at any size
+@pytest.mark.parametrize("op,les,layout,whole", [
+    ("reg", True, (208, 104, 104), True), ("reg", True, (240, 120, 120), False), ("trt", True, (240, 120, 120), True),
+    ("reg", False, (288, 144, 144), True), ("reg", False, (336, 168, 168), False)])
+def test_large_binary32_steps_are_split(op, les, layout, whole):
+    """profile_steps gives a step of one launch whole; the values are those of a shared domain's
+    split step either way."""
+    from pocketwind_gb300 import meshes
+    G, S = _pw()
+    grid = G.voxelize(meshes.icosphere([n / 2.1 for n in layout], 9.3, 3), None, layout, True)
+    got = []
+    for shared in (False, True):
+        s = S.GpuSolver.create(layout, grid, S.SolverParams(tau0=0.56, u_in=0.05, les=les, operator=op))
+        s.share(shared)
+        ms = s.profile_steps(2)
+        assert (ms[1] == 0) == (whole and not shared), ms
+        s.step(5, True)
+        got.append(s.macros())
+        s.destroy()
+    assert np.array_equal(*got)
