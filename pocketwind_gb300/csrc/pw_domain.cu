@@ -648,8 +648,6 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   a.want((void **)&d->macros, cells * sizeof(float4));
   a.want((void **)&d->flags, cells * 4);
   a.want((void **)&d->special, ((cells + 31) / 32 + 1) * 4);
-  uint32_t *edge_counts = nullptr;
-  if (!d->tiled && !desc->strict) a.want((void **)&edge_counts, edge_count_words((uint32_t)cells) * 4);
   d->interp = desc->walls == PW_WALLS_BOUZIDI;
   if (d->interp) {
     a.want((void **)&d->qoff, cells * 4);
@@ -665,6 +663,8 @@ int pw_domain_create(const pw_domain_desc *desc, const pw_grid *grid, pw_domain 
   a.want((void **)&d->status_dev, 16);
   a.want((void **)&d->tiles_taken, sizeof(uint32_t));
   a.want((void **)&d->totals_dev, 4 * sizeof(double));
+  uint32_t *edge_counts = nullptr;
+  if (!d->tiled && !desc->strict) a.want((void **)&edge_counts, edge_count_words((uint32_t)cells) * 4);
   prepare_pool();
   if (e == cudaSuccess) e = a.alloc(&d->arena);
   if (e == cudaSuccess) {
