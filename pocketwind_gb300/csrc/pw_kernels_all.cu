@@ -16,7 +16,8 @@ extern template void launch_storage<STORE_BF16>(const StepParams &, int, int, bo
 // and 74.2, BF16 there 73.0 and 74.1, 320x160x160 136.2 and 139.6; FP16 TRT 224x112x112
 // 53.3 and 54.5, 300x150x150 113.6 and 119.3): past that the side kernels' own register
 // counts pay more than the launches cost; and not beside reflecting seam rows, which take
-// one cell a thread.  16-bit storage with nx odd: any size (203x101x67 without LES
+// one cell a thread (with nx even only the split step is built and measured for them: a
+// free-slip FP16 TRT sphere 96x48x48 20.1 us a step in calls of 8, 14.2 in captured runs).  16-bit storage with nx odd: any size (203x101x67 without LES
 // 35.0 and 24.4, 399x200x200 308 and 266; FP16 REG with LES 97x48x48 25.4 and 15.9,
 // 203x101x101 48.5 and 37.2, 399x199x199 299 and 266; free-slip BF16 97x48x48 59 and
 // 17), but FP16 TRT with LES: the compiler rounds that seam's rows differently in this
