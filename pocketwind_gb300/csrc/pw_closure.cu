@@ -1316,11 +1316,17 @@ static void closure_pairs_step(const StepParams &p, const uint32_t *frag, const 
 // edge cells the line is later (a sphere without a floor, FP16: 72x36x36 18.5 and 15.8,
 // 73x37x37 18.7 and 16.8, 88x44x44 18.0 and 19.7).  With the floor layer in a kernel of its
 // own the early launches are the faster ones at any size (FP16 64x32x32 16.1 and 16.3).
-bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int floor_rows, uint32_t count) {
+// FP32 TRT with many edge cells (a floor) is faster captured again once the tiles fill the
+// GPU: 97x49x49 29.0 and 28.4, 104x52x52 31.6 and 30.0, 128x64x64 42.1 and 41.0, 160x80x80
+// 81.5 and 77.0; REG is not (97x49x49 24.0 and 24.7, 128x64x64 34.5 and 35.9).
+bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int op, int floor_rows,
+                                uint32_t count) {
   if (floor_rows && ny >= 3u) return false;
   const uint64_t tiles = (uint64_t)((nx + 63u) / 64u) * ((ny + 3u) / 4u) * nz, sms = (uint64_t)multiprocessors();
   const uint64_t edge = (count + pwclosure::NTHREADS - 1) / pwclosure::NTHREADS;
-  return 5u * tiles <= (8u * edge < sms ? 25u : 21u) * sms;
+  const bool many = 8u * edge >= sms;
+  return 5u * tiles <= (many ? 21u : 25u) * sms ||
+         (storage == pw::STORE_F32 && op == pw::OP_TRT && many && tiles >= 8u * sms);
 }
 
 void launch_closure_pairs(const StepParams &p, int storage, int op, bool odd, const uint32_t *frag,

@@ -767,7 +767,8 @@ int pw_step(pw_domain *d, uint64_t count, int write_macro_on_last) {
   // 192x96x96 FP16 45.9 us a step against 37.9; 128x64x64 24.0 against 28.9).
   const bool closure_graphs =
       d->closure_frag && d->split &&
-      pwclosure_host::closure_long_runs_captured(d->nx, d->ny, d->nz, d->floor_rows, d->edge_own);
+      pwclosure_host::closure_long_runs_captured(d->nx, d->ny, d->nz, d->desc.storage, d->desc.op, d->floor_rows,
+                                                 d->edge_own);
   const bool use_graphs =
       closure_graphs || (!single_launch(d) && d->cells <= (size_t)(d->split ? 1 : 8) << 20);
   uint64_t past_graphs = 0;  // a captured step clears no guard flag for the one behind it

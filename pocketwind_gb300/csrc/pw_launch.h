@@ -88,7 +88,8 @@ void launch_closure_pairs(const pw::StepParams &p, int storage, int op, bool odd
                           const uint8_t *wall, const uint32_t *list, uint32_t count, uint32_t *taken, bool early,
                           cudaStream_t s, const pwfast::SideStream *side = nullptr);
 // Whether a long run of such steps is faster captured, with side, than launched early.
-bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int floor_rows, uint32_t count);
+bool closure_long_runs_captured(uint32_t nx, uint32_t ny, uint32_t nz, int storage, int op, int floor_rows,
+                                uint32_t count);
 int wall_distance_of(const uint32_t *flags, uint32_t nx, uint32_t ny, uint32_t nz, uint8_t *out, cudaStream_t s);
 const uint32_t *fragments(const pw_closure *c);
 }

@@ -336,18 +336,21 @@ def test_trained_closure_beats_smagorinsky_on_held_out_data():
 
 
 # sizes whose long runs are captured (64 steps a graph) and, the last, one past the line;
-# 65 and 129 steps leave one step behind the graphs
+# 65 and 129 steps leave one step behind the graphs; with 1,352 tiles the captured blocks
+# take theirs from the counter
 @pytest_gpu
-@pytest.mark.parametrize("precision,layout", [("f32", (64, 32, 32)), ("f16", (33, 17, 17)), ("f32", (72, 36, 36))])
+@pytest.mark.parametrize("precision,operator,layout", [
+    ("f32", "reg", (64, 32, 32)), ("f16", "reg", (33, 17, 17)), ("f32", "trt", (104, 52, 52)),
+    ("f32", "reg", (72, 36, 36))])
 @pytest.mark.parametrize("count", [64, 65, 129])
-def test_long_closure_runs_equal_single_steps(precision, layout, count):
+def test_long_closure_runs_equal_single_steps(precision, operator, layout, count):
     from pocketwind_gb300 import geometry, meshes, solver
     net = _closure(_rand_params(9))
     grid = geometry.voxelize(meshes.icosphere([n / 2.2 for n in layout], min(layout) / 5, 3), None, layout, True)
     got = []
     for calls in ([1] * count, [count]):
-        s = solver.GpuSolver.create(layout, grid, solver.SolverParams(tau0=0.56, u_in=0.05, les=True, operator="reg",
-                                                                      precision=precision))
+        s = solver.GpuSolver.create(layout, grid, solver.SolverParams(tau0=0.56, u_in=0.05, les=True,
+                                                                      operator=operator, precision=precision))
         net.attach(s)
         s.inject_nan()
         s.step(1, True)
